@@ -155,7 +155,6 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 MB_API int mb_gemm_f32(const float* A, const float* W, float* C, int N, int M, int K, int ldc, cudaStream_t st) {
     if (N == 0 || M == 0) return 0;
     if (ldc < M) return -2;
-    if ((N + 15) / 16 > 65535) return -2;
     const bool vec = K % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
     auto tiles = [&](int bm, int bn) { return (long long)((N + bm - 1) / bm) * ((M + bn - 1) / bn); };
     // The largest tile that still gives every SM its four blocks, since it reads the operands least; measured (us, 128 x 64 /
@@ -163,6 +162,8 @@ MB_API int mb_gemm_f32(const float* A, const float* W, float* C, int N, int M, i
     // most SMs idle, 149 / 128 / 149 / 184; 17 x 16384 x 2048 218 / 126 / 101 / 107; 130 x 2048 x 2048 145 / 81 / 91 / 62;
     // 1 x 128256 x 2048 1254 / 726 / 466 / 336.  (One tile of 64 x 64 for all, without a stage ahead: 1353, 219, 226, 156, 1159.)
     const int t = N <= 16 ? 3 : tiles(128, 64) >= 592 ? 0 : N > 32 && tiles(64, 64) >= 148 ? 1 : N <= 32 && tiles(32, 64) >= 148 ? 2 : 3;
+    const int rows[4] = {128, 64, 32, 16};
+    if (((long long)N + rows[t] - 1) / rows[t] > 65535) return -2;
 #define GF_CASE(ID, BM, BN, TM, TN)                                                                                        \
     if (t == ID) {                                                                                                         \
         const dim3 grid((M + BN - 1) / BN, (N + BM - 1) / BM);                                                             \

@@ -34,6 +34,15 @@ def test_gemm_f32_tiles_give_the_bits_of_a_row_alone(N, M, Kd, off):
     assert bool((out._base[:, M:] == 7.0).all())
 
 
+def test_gemm_f32_takes_more_rows_than_the_smallest_tile_could():
+    K = ops()
+    N, M, Kd = 16 * 65535 + 17, 5, 3
+    a, w = torch.randn(N, Kd, device=G.DEV), torch.randn(M, Kd, device=G.DEV)
+    out = K.linear(a, w)
+    bound = (a.abs().double() @ w.abs().double().T) * Kd * 2.0 ** -24 + 1e-30
+    assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all())
+
+
 # (lengths, tokens of the step): runs that fill tiles, straddle them, are too short for the tiled form, stand on their edges
 @pytest.mark.parametrize("H,KV,HD,HDV,page,lengths,q_lens", [
     (32, 8, 64, 64, 16, [100, 40, 33], [100, 1, 33]),
