@@ -156,14 +156,23 @@ MB_API int mb_gemm_f32(const float* A, const float* W, float* C, int N, int M, i
     if (N == 0 || M == 0) return 0;
     if (ldc < M) return -2;
     const bool vec = K % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
-    auto tiles = [&](int bm, int bn) { return (long long)((N + bm - 1) / bm) * ((M + bn - 1) / bn); };
-    // The largest tile that still gives every SM its four blocks, since it reads the operands least; measured (us, 128 x 64 /
-    // 64 x 64 / 32 x 64 / 16 x 64): 509 x 16384 x 2048 685 / 771 / 965 / 1329; 509 x 2048 x 2048, where the first leaves
-    // most SMs idle, 149 / 128 / 149 / 184; 17 x 16384 x 2048 218 / 126 / 101 / 107; 130 x 2048 x 2048 145 / 81 / 91 / 62;
-    // 1 x 128256 x 2048 1254 / 726 / 466 / 336.  (One tile of 64 x 64 for all, without a stage ahead: 1353, 219, 226, 156, 1159.)
-    const int t = N <= 16 ? 3 : tiles(128, 64) >= 592 ? 0 : N > 32 && tiles(64, 64) >= 148 ? 1 : N <= 32 && tiles(32, 64) >= 148 ? 2 : 3;
+    auto padded = [&](int bm) { return ((long long)N + bm - 1) / bm * bm; };
+    auto tiles = [&](int bm, int bn) { return padded(bm) / bm * ((M + bn - 1) / bn); };
+    // The largest tile that still gives every SM its four blocks, since it reads the operands least (64 rows of the first cost
+    // what 56 of the second do), unless its padding costs more than that; measured (us, 128 x 64 / 64 x 64 / 32 x 64 /
+    // 16 x 64): 509 x 16384 x 2048 688 / 770 / 966 / 1330; 160 x 32000 x 2048, where the first has 256 rows and the second
+    // 192, 674 / 606 / 629 / 817; 509 x 2048 x 2048, where the first leaves most SMs idle, 145 / 131 / 150 / 190; the head of
+    // 128,256 columns (K 2,048): 128 rows 1329 / 1511 / 1911 / 2593, 65 rows 1288 / 1468 / 1413 / 1599, 64 rows 1288 / 774 /
+    // 967 / 1332, 33 rows 1268 / 748 / 942 / 993, 32 rows 1266 / 748 / 496 / 678, 17 rows 1262 / 737 / 481 / 664, one row
+    // 1253 / 729 / 469 / 336; 17 x 16384 x 2048 219 / 129 / 109 / 111; 130 x 2048 x 2048 145 / 81 / 91 / 62.  (One tile of
+    // 64 x 64 for all, without a stage ahead: 1355, 1053, 227, 2678, 2464, 1360, 1257, 1257, 1206, 1158, 225, 156.)
+    const int t = N <= 16                                                        ? 3
+                  : tiles(128, 64) >= 592 && 7 * padded(128) <= 8 * padded(64) ? 0
+                  : N > 32 && tiles(64, 64) >= 148                             ? 1
+                  : N <= 32 && tiles(32, 64) >= 148                            ? 2
+                                                                               : 3;
     const int rows[4] = {128, 64, 32, 16};
-    if (((long long)N + rows[t] - 1) / rows[t] > 65535) return -2;
+    if (padded(rows[t]) / rows[t] > 65535) return -2;
 #define GF_CASE(ID, BM, BN, TM, TN)                                                                                        \
     if (t == ID) {                                                                                                         \
         const dim3 grid((M + BN - 1) / BN, (N + BM - 1) / BM);                                                             \

@@ -34,6 +34,12 @@ def test_gemm_f32_tiles_give_the_bits_of_a_row_alone(N, M, Kd, off):
     assert bool((out._base[:, M:] == 7.0).all())
 
 
+@pytest.mark.parametrize("N", [17, 32, 33, 64, 65, 128, 129, 192, 193])
+def test_gemm_f32_many_columns(N):
+    """more than 592 tiles of 64 columns: the rows decide the tile"""
+    test_gemm_f32_tiles_give_the_bits_of_a_row_alone(N, 37889, 20, 0)
+
+
 def test_gemm_f32_takes_more_rows_than_the_smallest_tile_could():
     K = ops()
     N, M, Kd = 16 * 65535 + 17, 5, 3
