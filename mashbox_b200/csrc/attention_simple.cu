@@ -14,8 +14,9 @@
 #define SIMPLE_MAX_HD 1024         // the widest rows (three instantiations: up to 256, up to 512, and up to this)
 #define WARPS 4
 
-// Which tokens the tiled form (below) takes: the step's tokens are looked at in tiles of `tile` neighbours; a run of at least SIMPLE_RUN tokens of one sequence inside a tile is the tiled
-// form's, the others -- decoded tokens, the ends of short portions -- are the plain form's.  Both forms compute the same bits.
+// Which tokens the tiled form (below) takes: the step's tokens are looked at in tiles of `tile` neighbours; a run of at least
+// SIMPLE_RUN neighbours inside a tile that are tokens of one sequence in order is the tiled form's, the others -- decoded tokens,
+// the ends of short portions, tokens in any other order -- are the plain form's.  Both forms compute the same bits.
 #define SIMPLE_RUN 4
 __device__ __forceinline__ bool simple_same(const int* __restrict__ tok_seq, const int* __restrict__ positions, int j, int n) {
     return tok_seq[j] == tok_seq[n] && positions[j] - positions[n] == j - n;
@@ -34,10 +35,13 @@ __global__ void __launch_bounds__(WARPS * 32) attn_simple_kernel(
     if (item >= (long long)N * H) return;
     const int n = (int)(item / H), h = (int)(item % H);
     if (tile) {
-        const int t0 = n - n % tile, t1 = min(t0 + tile, N);
-        int same = 0;
-        for (int j = t0 + lane; j < t1; j += 32) same += simple_same(tok_seq, positions, j, n);
-        if (__reduce_add_sync(0xffffffffu, same) >= SIMPLE_RUN) return;
+        // the run around n: its tokens stand side by side (a tile has at most 64)
+        const int t0 = n - n % tile, t1 = min(t0 + tile, N), i = n - t0;
+        const bool lo = t0 + lane < t1 && simple_same(tok_seq, positions, t0 + lane, n);
+        const bool hi = t0 + 32 + lane < t1 && simple_same(tok_seq, positions, t0 + 32 + lane, n);
+        const unsigned long long same = __ballot_sync(0xffffffffu, lo) | (unsigned long long)__ballot_sync(0xffffffffu, hi) << 32;
+        const unsigned long long after = ~(same >> i), before = i ? ~(same << (64 - i)) : ~0ull;       // zeros: the run's
+        if ((after ? __ffsll(after) - 1 : 64) + __clzll(before) >= SIMPLE_RUN) return;
     }
     const int kvh = h / (H / KV);
     const int pos = positions[n];
@@ -111,10 +115,10 @@ __global__ void __launch_bounds__(WARPS * 32) attn_simple_kernel(
 // The tiled form, float32, every key from position 0 on: a block is a run of tokens of one sequence (up to 64 / HB of them)
 // times HB query heads of one kv head, 64 rows that read the same keys.  The plain form reads every key once for every
 // row, one float at a time; here a tile of 32 keys and values is brought to shared memory once for the 64 rows, and the two
-// products are register-tiled (4 rows x 4 keys, 4 rows x HDV / 8 values a thread), the next tile on its way meanwhile.  The arithmetic of a
-// row is the plain form's, operation by operation and in its order -- scores by fused multiply-adds in ascending channel,
-// 32 keys to a step of the softmax counted from position 0, the weights met by the same tree, values added in ascending
-// key --, so the two forms give the same bits and a prompt's logits do not depend on how it was cut.
+// products are register-tiled (4 rows x 4 keys, 4 rows x HDV / 8 values a thread), the next tile on its way meanwhile.
+// The arithmetic of a row is the plain form's, operation by operation and in its order -- scores by fused multiply-adds in
+// ascending channel, 32 keys to a step of the softmax counted from position 0, the weights met by the same tree, values added
+// in ascending key --, so the two forms give the same bits and a prompt's logits do not depend on how it was cut.
 // 509 tokens of 32 heads of 64 (8 kv heads): 1,338 us in the plain form, 123 here; 24 heads of 128: 1,824 and 190.
 #define ST_ROWS 64
 #define ST_KEYS 32
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(ST_THREADS) attn_simple_tiled_kernel(
     int k_row, int v_row, float softcap, const float* __restrict__ sinks, const float* __restrict__ gate, int gate_stride,
     int HB, int tile) {
     constexpr int RS = ST_ROWS + 4, VS = 32 * DG;
-    const int KS = HD + 4 + (HD & 4 ? 4 : 0);       // a multiple of 4 that is an odd number of quads at HD = 64, 128, ..: eight keys on eight banks of quads
+    const int KS = HD + 4 + (HD & 4 ? 4 : 0);       // an odd number of quads at HD = 64, 128, ..: eight keys on eight banks of quads
     extern __shared__ __align__(16) float st_smem[];
     float* Qs = st_smem;                    // [HD][RS]
     float* Ps = Qs + HD * RS;               // [ST_KEYS][RS]: weights, key by key

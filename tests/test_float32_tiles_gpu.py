@@ -90,3 +90,30 @@ def test_tiled_attention_gives_the_bits_of_the_plain_form(H, KV, HD, HDV, page, 
     assert torch.equal(whole, torch.cat([run(n, n + 1) for n in range(seqs.N)]))
     seqs.table = table
     err.zero_()
+
+
+@pytest.mark.parametrize("order", ["gaps", "reversed", "shuffled", "whole"])
+def test_tokens_in_any_order_are_all_computed(order):
+    """The tiled form takes runs of neighbours that are one sequence's tokens in order; every other token is the plain form's --
+    also one whose neighbours beyond another sequence's token would continue it ("gaps": three tokens, one of another sequence,
+    three tokens, each at the place its position asks for)."""
+    K = ops()
+    H, KV, HD, page = 8, 2, 64, 16
+    seqs = G.PagedSequences([120, 60], [120, 60], H, KV, HD, page, torch.float32, seed=3).round().build()
+    places = list(range(seqs.N))
+    if order == "gaps":
+        places = [120 + j // 4 if j % 4 == 3 else j for j in range(120)]
+    elif order == "reversed":
+        places = places[::-1]
+    elif order == "shuffled":
+        places = torch.randperm(seqs.N, generator=torch.Generator().manual_seed(1)).tolist()
+    err, at = K.new_error_word(G.DEV), torch.tensor(places, device=G.DEV)
+
+    def run(at):
+        out = torch.full((len(at), H * HD), 7.0, device=G.DEV)
+        K.attention_simple(seqs.q_dev[at].contiguous(), H * HD, out, seqs.positions[at].contiguous(), seqs.tok_row[at].contiguous(),
+                           seqs.table, seqs.kpool, seqs.vpool, H, KV, HD, page, seqs.num_pages, None, HD ** -0.5, err)
+        return out
+    alone = torch.cat([run(at[n:n + 1]) for n in range(len(places))])
+    assert torch.equal(run(at), alone)
+    K.check_error_word(err)
