@@ -476,15 +476,17 @@ __global__ void __launch_bounds__(256) chunk_walk_kernel(const float* __restrict
                 }
             }
     } else {
+        int sent = min(LC_STAGES, chunks);                       // records sent for (thread 128)
         for (int c = 0; c < chunks; c++) {
             const int buf = c & 1, at_stage = c % LC_STAGES;
             const float* record = sm + at_stage * R::ALL;
             const float* second = record + R::FIRST;
             // A has taken the chunk before this one in, and all of B is done with it: its record's buffer is free
             lc_wait<LC_S_READY>(buf);
-            if (threadIdx.x == 128 && c > 0 && c - 1 + LC_STAGES < chunks) {
+            if (threadIdx.x == 128 && c > 0 && c - 1 + LC_STAGES < chunks && !bad) {
                 const int free = (c - 1) % LC_STAGES;
                 lc_fetch(sm + free * R::ALL, rec + (size_t)(c - 1 + LC_STAGES) * next, R::ALL * 4, bar0 + 8 * free);
+                sent = c + LC_STAGES;
             }
             if (!bad) bad = !mbar_wait(bar0 + 8 * at_stage, (c / LC_STAGES) & 1, err);
             lc_rows<SLAB>(record + warp * SLAB * R::ROWS, R::ROWS, sS + (size_t)(buf * DP + warp * SLAB) * LC_COLS,
@@ -496,6 +498,9 @@ __global__ void __launch_bounds__(256) chunk_walk_kernel(const float* __restrict
             lc_lower(out, second + R::A, sU + buf * LC_C * LC_COLS, tt, last, cg);
             if (colin && c * LC_C + tt < len) *reinterpret_cast<float4*>(o + vat + (size_t)c * vnext) = out;
         }
+        // a wait ran out: the block does not leave while copies into its shared memory may still be on their way
+        if (threadIdx.x == 128 && bad)
+            for (int r = max(0, sent - LC_STAGES); r < sent; r++) mbar_wait(bar0 + 8 * (r % LC_STAGES), (r / LC_STAGES) & 1, err);
     }
 }
 
