@@ -1289,12 +1289,6 @@ def attention_tma_merges(n_items, KV):
     return n_items * KV <= MERGE_COUNTERS
 
 
-def attention_tma_merges_uneven(n_items, KV):
-    """True when the sequences of a launch may be cut into different numbers of splits, with items that hold no rows among
-    them: the kernel merges the splits itself, group by group"""
-    return attention_tma_merges(n_items, KV)
-
-
 def attention_tma_folds_rotation(G):
     """True when attention_tma can take the rotate-and-store step of a step of one-token sequences in (rope=...)"""
     return 1 <= G <= 16

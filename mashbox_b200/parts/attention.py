@@ -181,26 +181,27 @@ class PagedAttention:
                 crowd = many_splits(base[True], work, slots, self.HD, min(4, max_splits))
         # Sequences of very different lengths, cut into equally many splits, leave the launch waiting for the blocks of the
         # longest one.  They are cut in proportion instead (3B shape, 37 sequences of 128 to 4,096 tokens: a step 3,600 ->
-        # 3,250 us; 11 of them beside a prompt of 1,499: 10,250 -> 10,050).  The work list is as long as the number of sequences says -- empty items fill it up -- so that
+        # 3,250 us; 11 of them beside a prompt of 1,499: 10,250 -> 10,050).  The work list is as long as the number of
+        # sequences says -- empty items fill it up -- and every token has a place in the partial buffers, split or not, so that
         # growing sequences do not change a step's shape.
         uneven, slots = {}, 0
         decoding = [s for s in range(S) if decode_form[s]]
-        takes = getattr(ctx.ops, "attention_tma_merges_uneven", None)
-        if (takes is not None and len(decoding) > 1 and self._tma(ctx) and ctx.options.get("attention_splits") is None
+        if (len(decoding) > 1 and self._tma(ctx) and ctx.options.get("attention_splits") is None
                 and ctx.options.get("attention_cluster_size") is None and ctx.options.get("attention_fused_merge", True)
                 and ctx.options.get("attention_uneven_splits", True)):
             lengths = [key_tiles(s) for s in decoding]
             slots = 2 * ctx.ops.attention_tma_active_clusters(self.HD, 2)
             items = max(2 * len(decoding), -(-3 * slots // KV))
             if (slots and 2 * max(lengths) * len(decoding) >= 3 * sum(lengths)
-                    and takes(items + max_splits * S + sum(tiles), KV)):
+                    and ctx.ops.attention_tma_merges(items + max_splits * S + sum(tiles), KV)):
                 uneven = dict(zip(decoding, uneven_splits(lengths, items, max_splits)))
                 cluster = 0
         for s in range(S):
             kv_tiles = key_tiles(s)
             ns = 1
             if s in uneven:
-                part_base[s] = len(part_tok) // 2
+                if uneven[s] > 1:
+                    part_base[s] = len(part_tok) // 2
                 for t in range(ctx.q_len[s]):
                     part_tok += [ctx.q_start[s] + t, uneven[s]]
                 dec += [(0, s, 0, sp, uneven[s]) for sp in range(uneven[s])]
@@ -235,7 +236,7 @@ class PagedAttention:
         ctx.inputs.add(name + "part_base", np.asarray(part_base, np.int32))
         ctx.inputs.add(name + "part_tok", np.asarray(part_tok, np.int32))
         ctx.memo[key] = dict(name=name, n_dec=len(dec), n_pre=len(pre), n_mid=len(mid), n_part=len(part_tok) // 2,
-                             max_splits=max_splits, tc5=tc5, cluster=cluster)
+                             max_splits=max_splits, tc5=tc5, cluster=cluster, uneven=bool(uneven))
 
     # ------------------------------------------------------------------------------------------ kernels
     def attend(self, ctx, qkv, width, out, table, kpool, vpool, rope=None, sinks=None, gate=None):

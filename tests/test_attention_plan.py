@@ -22,6 +22,7 @@ class FakeOps:
     def attention_tma_supports(self, HD, page): return True
     def attention_tma_max_cluster(self, HD): return 8
     def attention_tma_active_clusters(self, HD, c): return ACTIVE[c]
+    def attention_tma_merges(self, n, KV): return n * KV <= 1 << 16
 
 
 class Inputs(dict):
@@ -44,7 +45,11 @@ def plan(lengths, new, options=None, heads=32, kv=8, window=None):
 
 def check_cover(p, dec, pre, part_base, part_tok, lengths, new, G=4):
     seen = {}
-    for s, m, sp, ns in list(dec) + list(pre):
+    uneven = p["uneven"]
+    real = [r for r in dec if r[1] == 0]                # the other items of an uneven plan are empty: a row tile beyond all rows
+    assert uneven or len(real) == len(dec)
+    assert all(r[1] * 16 >= 1 << 20 and r[3] == 1 for r in dec if r[1])
+    for s, m, sp, ns in real + list(pre):
         seen.setdefault((s, m), []).append((sp, ns))
     for s, (n, q) in enumerate(zip(lengths, new)):
         tiles = [k for k in seen if k[0] == s]
@@ -53,14 +58,20 @@ def check_cover(p, dec, pre, part_base, part_tok, lengths, new, G=4):
             ns = seen[k][0][1]
             assert sorted(sp for sp, _ in seen[k]) == list(range(ns)) and all(x == ns for _, x in seen[k])
             assert ns <= max(1, -(-n // KEY_TILE) // 2) or ns == 1 or p["cluster"]
+            if uneven and q * G <= 16:                  # at least 4 key tiles a split, and side by side (the merge counts from the first)
+                first = [r[0] for r in dec].index(s)
+                assert ns <= max(1, -(-n // (4 * KEY_TILE))) and [r[0] for r in dec[first:first + ns]] == [s] * ns
             assert (part_base[s] >= 0) == (ns > 1 and not (p["cluster"] and q * G <= 16))
     if p["cluster"]:
         c = p["cluster"]
         assert len(dec) % c == 0
         for i in range(0, len(dec), c):                               # a cluster is the splits of one sequence, in order
             assert [tuple(r) for r in dec[i:i + c]] == [(dec[i][0], 0, sp, c) for sp in range(c)]
-    # the partial buffers: one place per token of a split sequence
-    assert len(part_tok) == sum(q for s, q in enumerate(new) if part_base[s] >= 0)
+    # the partial buffers: one place per token of a split sequence (an uneven plan: of every decode-form sequence)
+    assert len(part_tok) == sum(q for s, q in enumerate(new) if part_base[s] >= 0 or uneven and q * G <= 16)
+    for s, q in enumerate(new):
+        if part_base[s] >= 0:
+            assert [r[0] for r in part_tok[part_base[s]:part_base[s] + q]] == [sum(new[:s]) + t for t in range(q)]
 
 
 @pytest.mark.parametrize("batch,keys", [(1, 8192), (2, 8192), (3, 8192), (4, 8192), (5, 8192), (8, 8192), (11, 8192),

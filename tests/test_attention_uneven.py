@@ -10,24 +10,20 @@ from mashbox_b200.parts import attention as A
 from tests import test_attention_plan as T
 
 
-class Ops(T.FakeOps):
-    def attention_tma_merges_uneven(self, n, KV): return n * KV <= 1 << 16
-
-
-def test_every_key_tile_once_and_as_many_items_as_the_sequences_say(monkeypatch):
-    monkeypatch.setattr(T, "FakeOps", Ops)
+def test_every_key_tile_once_and_as_many_items_as_the_sequences_say():
     rng = random.Random(3)
     used = 0
     for _ in range(300):
-        S, kv = rng.randint(2, 70), rng.choice([1, 4, 8])
+        S, kv = rng.randint(2, 70), rng.choice([2, 4, 8])
         lengths = [rng.choice([1, 2, 63, 64, 65, 500, 4096, 20000]) for _ in range(S)]
         new = [1] * S if rng.random() < 0.5 else [min(n, rng.choice([1, 1, 4, 700])) for n in lengths]
         p, dec, pre, part_base, part_tok = T.plan(lengths, new, kv=kv, window=rng.choice([None, None, 1000]))
         rows = [s for s, _, _, _ in dec]
         real = [tuple(r) for r in dec if r[1] == 0]
         decoding = [s for s, q in enumerate(new) if q * (32 // kv) <= 16]
-        if p["cluster"] or not decoding or len(real) == len(dec) and len(part_tok) < len(decoding):
+        if not p["uneven"]:
             continue
+        T.check_cover(p, dec, pre, part_base, part_tok, lengths, new, 32 // kv)
         by = {s: [(sp, ns) for t, _, sp, ns in real if t == s] for s in decoding}
         assert all(by[s] == [(i, len(by[s])) for i in range(len(by[s]))] and 1 <= len(by[s]) <= 32 for s in decoding)
         if len(dec) > len(real):
@@ -71,10 +67,10 @@ def test_uneven_splits_give_the_logits_of_equal_ones(name, tmp_path):
                 step.append(("p", ids[0][:77], [76]))
             ctx = eng.runner.prepare(step)
             plan = next(v for k, v in ctx.memo.items() if k[0] == "attention")
-            used.append(plan["n_dec"] > 5 * max(1, plan["cluster"]))
+            used.append(plan["uneven"])
             got.append(eng.runner.launch(ctx, step).float().cpu().clone())
         eng.runner.check()
         outs.append(torch.cat(got))
-    assert all(used[:4])
+    assert used == [True] * 4 + [False] * 4
     err = float((outs[0] - outs[1]).norm() / outs[1].norm())
     assert err < 1e-2, err
