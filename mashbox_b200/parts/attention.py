@@ -54,6 +54,14 @@ def uneven_splits(tiles, items, most):
     return [max(1, min(most, -(-t // 4), t * (items - len(tiles)) // work)) for t in tiles]
 
 
+def listed_items(real):
+    """the length of a work list of `real` items: the next of 4, 6, 8, 12, 16, 24, ..."""
+    n = 4
+    while n < real:
+        n = n * 3 // 2 if n & (n - 1) == 0 else n * 4 // 3
+    return n
+
+
 class PagedAttention:
     """Attention of a step's queries over rows kept per position in pages: the work lists (`prepare`, on the host) and
     the choice of kernel (`attend`).  `heads` query heads read `kv_heads` rows of `head_dim` values per position;
@@ -137,6 +145,7 @@ class PagedAttention:
         # token is already a prompt-form tile, which the tcgen05 kernel does not cut along the keys.  Such stretches of
         # at most DECODE_ROWS tokens go to the TMA/mma prompt form with splits, in a list of their own.
         wide = tc5 and G > DECODE_ROWS
+        short = lambda s: wide and not decode_form[s] and ctx.q_len[s] <= DECODE_ROWS
 
         def key_tiles(s):
             hi = ctx.pos0[s] + ctx.q_len[s]
@@ -179,26 +188,42 @@ class PagedAttention:
             if slots and 2 * base[True] > slots:
                 work = sum(key_tiles(s) for s in range(S) if decode_form[s]) * KV
                 crowd = many_splits(base[True], work, slots, self.HD, min(4, max_splits))
+        def even_splits(s):
+            if cluster and decode_form[s]:
+                return cluster
+            ns, kv_tiles = 1, key_tiles(s)
+            if ctx.q_len[s] <= DECODE_ROWS and base[decode_form[s]] < target and (decode_form[s] or not tc5 or short(s)):
+                ns = max(1, min(max_splits, -(-target // base[decode_form[s]]), kv_tiles // 2))
+                ns = 1 << (ns.bit_length() - 1)                    # a power of two: few distinct work-list shapes
+            if decode_form[s] and (crowd or ctx.options.get("attention_splits") is not None):
+                ns = max(1, min(crowd or int(ctx.options["attention_splits"]), kv_tiles // 2))
+            return ns
+
         # Sequences of very different lengths, cut into equally many splits, leave the launch waiting for the blocks of the
-        # longest one.  They are cut in proportion instead (3B shape, 37 sequences of 128 to 4,096 tokens: a step 3,600 ->
-        # 3,250 us; 11 of them beside a prompt of 1,499: 10,250 -> 10,050).  The work list is as long as the number of
-        # sequences says -- empty items fill it up -- and every token has a place in the partial buffers, split or not, so that
-        # growing sequences do not change a step's shape.
-        uneven, slots = {}, 0
+        # longest one; they are cut in proportion instead where that pays.  Measured on decode steps of 2 to 64 requests of
+        # 64 to 16,384 tokens (1B, 3B and 8B shapes, us a layer against the even plan):
+        #   * work for 16 tiles a slot of the device and more: in three rounds of blocks, faster wherever the longest block
+        #     gets shorter (40 requests of 64 to 4,096 tokens: -14; 64: -13; 24 of 64 to 16,384: -144);
+        #   * less: in one round, by how much shorter the longest block gets: by 6 tiles and more +0.1 to -200, by 5 from +0.3
+        #     to -2.9, by 4 and less +0.6 to +6 (splits that meet through global memory cost more than those of a cluster).
+        # The work list is filled up to a coarse grid of lengths with empty items, so that growing sequences seldom change a
+        # step's shape; for the same reason every token has a place in the partial buffers, split or not.
+        uneven = {}
         decoding = [s for s in range(S) if decode_form[s]]
-        if (len(decoding) > 1 and self._tma(ctx) and ctx.options.get("attention_splits") is None
-                and ctx.options.get("attention_cluster_size") is None and ctx.options.get("attention_fused_merge", True)
-                and ctx.options.get("attention_uneven_splits", True)):
+        choice = ctx.options.get("attention_uneven_splits", True)         # "always": without the look at what it brings
+        if (len(decoding) > 1 and choice and self._tma(ctx) and ctx.options.get("attention_splits") is None
+                and ctx.options.get("attention_cluster_size") is None and ctx.options.get("attention_fused_merge", True)):
             lengths = [key_tiles(s) for s in decoding]
             slots = 2 * ctx.ops.attention_tma_active_clusters(self.HD, 2)
-            items = max(2 * len(decoding), -(-3 * slots // KV))
-            if (slots and 2 * max(lengths) * len(decoding) >= 3 * sum(lengths)
-                    and ctx.ops.attention_tma_merges(items + max_splits * S + sum(tiles), KV)):
-                uneven = dict(zip(decoding, uneven_splits(lengths, items, max_splits)))
-                cluster = 0
+            if slots and 2 * max(lengths) * len(decoding) >= 3 * sum(lengths):
+                crowded = sum(lengths) * KV >= 16 * slots
+                cut = uneven_splits(lengths, max(2 * len(decoding), -(-(3 if crowded else 1) * slots // KV)), max_splits)
+                longest = lambda splits: max(-(-t // n) for t, n in zip(lengths, splits))
+                shorter = longest([even_splits(s) for s in decoding]) - longest(cut)
+                if ((choice == "always" or shorter >= (1 if crowded else 6))
+                        and ctx.ops.attention_tma_merges(max(listed_items(sum(cut)), max_splits * S + sum(tiles)), KV)):
+                    uneven, cluster = dict(zip(decoding, cut)), 0
         for s in range(S):
-            kv_tiles = key_tiles(s)
-            ns = 1
             if s in uneven:
                 if uneven[s] > 1:
                     part_base[s] = len(part_tok) // 2
@@ -206,27 +231,22 @@ class PagedAttention:
                     part_tok += [ctx.q_start[s] + t, uneven[s]]
                 dec += [(0, s, 0, sp, uneven[s]) for sp in range(uneven[s])]
                 continue
+            ns = even_splits(s)
             if cluster and decode_form[s]:
                 for sp in range(cluster):
                     dec.append((0, s, 0, sp, cluster))
                 continue
-            short = wide and not decode_form[s] and ctx.q_len[s] <= DECODE_ROWS
-            if ctx.q_len[s] <= DECODE_ROWS and base[decode_form[s]] < target and (decode_form[s] or not tc5 or short):
-                ns = max(1, min(max_splits, -(-target // base[decode_form[s]]), kv_tiles // 2))
-                ns = 1 << (ns.bit_length() - 1)                    # a power of two: few distinct work-list shapes
-            if decode_form[s] and (crowd or ctx.options.get("attention_splits") is not None):
-                ns = max(1, min(crowd or int(ctx.options["attention_splits"]), kv_tiles // 2))
             if ns > 1:
                 part_base[s] = len(part_tok) // 2
                 for t in range(ctx.q_len[s]):
                     part_tok += [ctx.q_start[s] + t, ns]
-            dst = dec if decode_form[s] else (mid if short else pre)
-            rows = PREFILL_ROWS if short else pre_rows
-            for m in range(-(-ctx.q_len[s] * G // rows) if short else tiles[s]):
+            dst = dec if decode_form[s] else (mid if short(s) else pre)
+            rows = PREFILL_ROWS if short(s) else pre_rows
+            for m in range(-(-ctx.q_len[s] * G // rows) if short(s) else tiles[s]):
                 for sp in range(ns):
                     dst.append((-(ctx.pos0[s] + (m + 1) * rows // G), s, m, sp, ns))
-        if uneven:
-            dec += [(0, decoding[0], 1 << 20, 0, 1)] * (items - len(dec))       # a row tile beyond the sequence's rows: empty
+        if uneven:                                                  # empty items: a row tile beyond the sequence's rows
+            dec += [(0, decoding[0], 1 << 20, 0, 1)] * (listed_items(len(dec)) - len(dec))
         pre.sort()                                                  # the tiles with the most keys first
         name = "attn%d_" % len([k for k in ctx.memo if k[0] == "attention"])
         flat = lambda items: np.asarray([i[1:] for i in items], np.int32).reshape(-1)

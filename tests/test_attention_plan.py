@@ -48,7 +48,7 @@ def check_cover(p, dec, pre, part_base, part_tok, lengths, new, G=4):
     uneven = p["uneven"]
     real = [r for r in dec if r[1] == 0]                # the other items of an uneven plan are empty: a row tile beyond all rows
     assert uneven or len(real) == len(dec)
-    assert all(r[1] * 16 >= 1 << 20 and r[3] == 1 for r in dec if r[1])
+    assert 2 * len(real) >= len(dec) and all(r[1] * 16 >= 1 << 20 and r[3] == 1 for r in dec if r[1])
     for s, m, sp, ns in real + list(pre):
         seen.setdefault((s, m), []).append((sp, ns))
     for s, (n, q) in enumerate(zip(lengths, new)):
