@@ -1601,15 +1601,18 @@ def gated_scan(q, k, v, g, o, state, seq, H, G, dim, vdim, per_head, bonus=None,
     _cuda(q, k, v, g, o, state, bonus, *seq)
     f = _fn("gated_scan", "mb_gated_scan", [c_void_p] * 7 + [c_ll] + [c_void_p] * 3 + [c_int] * 8 + [c_void_p])
     S = seq[0].shape[0]
-    # which layout of the state over threads: by the step's tokens per sequence (from the lengths of the arrays alone)
+    # which layout of the state over threads: by the step's tokens per sequence (from the lengths of the arrays alone); where
+    # long sequences are left alone, what counts is how many short ones run side by side (24 heads of 128 x 128 by channel
+    # beside 1,000 tokens, the layout for long stretches / for short ones: 63 sequences of a token 175 / 96 us, 16 of 20
+    # tokens 107 / 78, 2 of 31 tokens 31 / 23)
     _check(f(_p(q), _p(k), _p(v), _p(g), _p(bonus), _p(o), _p(state), state.stride(0), *[_p(t) for t in seq], S, H, G,
-             dim, vdim, 1 if per_head else 0, 1 if q.shape[0] > 4 * S else 0, int(below), _stream()), "gated_scan")
+             dim, vdim, 1 if per_head else 0, 1 if q.shape[0] > 4 * S and not below else 0, int(below), _stream()), "gated_scan")
 
 
 # ---- the linear-attention recurrences over long stretches, 32 tokens at a time (linear_chunks.cu).  A step runs them when it
 # has more than `tokens` tokens beyond one a sequence.  One sequence, 16 heads of 128 x 128, delta rule, chunks / scan: 65
 # tokens 34 / 28 us, 128 36 / 47, 512 75 / 168, 2,048 228 / 646.  Sequences of fewer than `shortest` tokens stay with the
-# scans, which then run beside the chunks' kernels.
+# scans, which then follow the chunks' kernels.
 CHUNKS = {"tokens": 80, "shortest": 32}
 CHUNK_MODES = {"delta": 0, "channels": 1, "heads": 2, "wkv": 3, "fixed": 4}
 

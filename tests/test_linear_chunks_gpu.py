@@ -158,6 +158,22 @@ def test_many_sequences_side_by_side(kind, lens):
     ops.check_error_word(ops.error_word(DEV))
 
 
+@pytest.mark.parametrize("kind", ("channels", "heads", "wkv"))
+def test_decoded_tokens_beside_a_prompt_run_as_without_it(kind):
+    """the scan of the short sequences lays the state out as it does in a step of theirs alone: the same bits"""
+    from mashbox_b200 import ops
+    H, dim, vdim, lens = 2, 128, 64, [200, 1, 2, 1]
+    N, n = sum(lens), H * dim * vdim
+    q, k, v, z, beta = inputs(kind, 9, N, H, H, dim, vdim, "slow")
+    start = (torch.randn(4, n, generator=torch.Generator().manual_seed(1)) * 0.1).to(DEV)
+    both, alone = start.clone(), start.clone()
+    o, p = torch.empty(N, H * vdim, device=DEV), torch.empty(4, H * vdim, device=DEV)
+    launch(ops, kind, True, q, k, v, z, beta, o, both, (i32([0, 200, 201, 203]), i32(lens), i32([0, 1, 2, 3])), H, H, dim, vdim)
+    launch(ops, kind, False, *(x[200:] for x in (q, k, v, z, beta)), p, alone, (i32([0, 1, 3]), i32(lens[1:]), i32([1, 2, 3])), H, H,
+           dim, vdim)
+    assert torch.equal(o[200:], p) and torch.equal(both[1:], alone[1:])
+
+
 def test_sizes_that_the_chunk_form_does_not_take():
     from mashbox_b200 import ops
     assert ops.linear_chunks_supports(2000, 3, 128, 64, "delta") and not ops.linear_chunks_supports(160, 80, 128, 64, "delta")
