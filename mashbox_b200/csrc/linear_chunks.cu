@@ -20,8 +20,8 @@
 //   chunk_walk   a block per sequence, head and 16 value columns walks the sequence's records in order with its part of
 //                S in registers.  Records come by bulk copy into two buffers of shared memory.
 //
-// A sequence of fewer than 32 tokens is passed over by both: a record of one token costs as much as one of 32 (16 sequences
-// of one token beside one of 64: 103 us against 46 by the scan).
+// A sequence of fewer than `shortest` tokens (32 at least) is passed over by both and left to the scan, which follows: a
+// record of one token costs as much as one of 32 (16 sequences of one token beside one of 64: 103 us against 46 by the scan).
 //
 // What bounds the walk is the shared-memory pipe: a lane takes one float a cycle, a thread's 4 x 4 tile needs eight for 16
 // multiply-adds, and the pipe is busy for 80 % of the cycles (delta rule, 16 heads of 128 x 128, 2,048 tokens: prep 46, walk
@@ -33,9 +33,9 @@
 
 #define LC_C 32                 // tokens of a chunk
 #define LC_COLS 16              // value columns of a walking block
-#define LC_STAGES 2             // records in shared memory (3 measured the same where one block has an SM to itself, and cost the second
-                                // block of an SM where it has not: 172 against 240 us on 24 heads)
-#define LC_MIN 32               // shorter sequences of a step are left to the token-by-token scan
+#define LC_STAGES 2             // records in shared memory (3 measured the same where one block has an SM to itself, and cost
+                                // the second block of an SM where it has not: 172 against 240 us on 24 heads)
+#define LC_MIN 32               // the least a sequence can be asked to have
 #define LC_RED 20               // floats a row of the partial sums takes (16 used; the padding keeps banks apart)
 
 // ---- pairs of floats: one issue slot, two results, each rounded as the single one is
@@ -70,13 +70,13 @@ struct Rec {
 };
 
 // chunks of a sequence
-__device__ __forceinline__ int lc_chunks(int len) { return len < LC_MIN ? 0 : (len + LC_C - 1) / LC_C; }
+__device__ __forceinline__ int lc_chunks(int len, int shortest) { return len < shortest ? 0 : (len + LC_C - 1) / LC_C; }
 
 // the sequence a slot (number of a chunk through all sequences in order) belongs to -> false beyond the last one
-__device__ __forceinline__ bool lc_find(int slot, int S, const int* __restrict__ q_len, int& s, int& c) {
+__device__ __forceinline__ bool lc_find(int slot, int S, const int* __restrict__ q_len, int shortest, int& s, int& c) {
     int base = 0;
     for (s = 0; s < S; s++) {
-        const int n = lc_chunks(q_len[s]);
+        const int n = lc_chunks(q_len[s], shortest);
         if (slot < base + n) { c = slot - base; return true; }
         base += n;
     }
@@ -88,7 +88,8 @@ template <int DP, int MODE>
 __global__ void __launch_bounds__(128) chunk_prep_kernel(const float* __restrict__ q, const float* __restrict__ k,
                                                          const float* __restrict__ g, const float* __restrict__ beta,
                                                          float* __restrict__ scratch, const int* __restrict__ q_start,
-                                                         const int* __restrict__ q_len, int S, int H, int G, int dim) {
+                                                         const int* __restrict__ q_len, int S, int H, int G, int dim,
+                                                         int shortest) {
     typedef Rec<DP, MODE> R;
     constexpr bool HEAD = MODE == 2 || MODE == 4;                // one decay per head
     constexpr int VEC = DP / 32;                                 // channels of a lane
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(128) chunk_prep_kernel(const float* __restrict
     float* sb = sB + (MODE == 0 ? LC_C * LC_C : 0);              // [32] beta, b, or a head's decays
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, j = h / (H / G);
     int s_, c_;
-    if (!lc_find(blockIdx.x, S, q_len, s_, c_)) return;
+    if (!lc_find(blockIdx.x, S, q_len, shortest, s_, c_)) return;
     const int n0 = q_start[s_] + c_ * LC_C, nb = min(LC_C, q_len[s_] - c_ * LC_C);
     float* rec = scratch + ((size_t)blockIdx.x * H + h) * R::ALL;
     auto fetch = [](float* d, const float* x) {
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(256) chunk_walk_kernel(const float* __restrict
                                                          float* __restrict__ state, long long state_stride,
                                                          const float* __restrict__ scratch, const int* __restrict__ q_start,
                                                          const int* __restrict__ q_len, const int* __restrict__ state_slot,
-                                                         int H, int dim, int vdim, int* err) {
+                                                         int H, int dim, int vdim, int shortest, int* err) {
     typedef Rec<DP, MODE> R;
     constexpr int SLAB = DP / 4, CH = DP / 32;
     extern __shared__ __align__(128) float sm[];
@@ -355,10 +356,10 @@ __global__ void __launch_bounds__(256) chunk_walk_kernel(const float* __restrict
     __shared__ __align__(8) uint64_t bars[LC_STAGES];
     const int tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31, rg = lane >> 2, cg = lane & 3;
     const int col0 = blockIdx.x * LC_COLS, h = blockIdx.y, sq = blockIdx.z;
-    const int a0 = q_start[sq], len = q_len[sq], chunks = lc_chunks(len);
+    const int a0 = q_start[sq], len = q_len[sq], chunks = lc_chunks(len, shortest);
     if (chunks == 0) return;
     int slot = 0;
-    for (int r = 0; r < sq; r++) slot += lc_chunks(q_len[r]);
+    for (int r = 0; r < sq; r++) slot += lc_chunks(q_len[r], shortest);
     const float* rec = scratch + ((size_t)slot * H + h) * R::ALL;
     const size_t next = (size_t)H * R::ALL;
     const uint32_t bar0 = smem_u32(bars);
@@ -507,11 +508,11 @@ __global__ void __launch_bounds__(256) chunk_walk_kernel(const float* __restrict
 template <int DP, int MODE>
 static int lc_launch(const float* q, const float* k, const float* v, const float* g, const float* beta, float* o, float* state,
                      long long state_stride, const int* q_start, const int* q_len, const int* state_slot, int S, int N, int H,
-                     int G, int dim, int vdim, float* scratch, long long scratch_floats, int* err, cudaStream_t st) {
+                     int G, int dim, int vdim, int shortest, float* scratch, long long scratch_floats, int* err, cudaStream_t st) {
     typedef Rec<DP, MODE> R;
     constexpr bool HEAD = MODE == 2 || MODE == 4;
-    // at least the sum of ceil(len / 32) over the sequences of 32 tokens and more, of which there are at most N / 32
-    const int slots = N / LC_C + (S < N / LC_C ? S : N / LC_C);
+    // at least the sum of ceil(len / 32) over the sequences of `shortest` tokens and more, of which there are at most N / shortest
+    const int slots = N / LC_C + (S < N / shortest ? S : N / shortest);
     if (slots == 0) return 0;
     if ((long long)slots * H * R::ALL > scratch_floats) return -2;
     const size_t smem1 = (size_t)(2 * LC_C * DP + (HEAD ? LC_C * LC_C : LC_C * DP) + (MODE == 0 ? 2 : 1) * LC_C * LC_C + LC_C) * 4;
@@ -526,11 +527,11 @@ static int lc_launch(const float* q, const float* k, const float* v, const float
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    chunk_prep_kernel<DP, MODE><<<dim3(slots, H), 128, smem1, st>>>(q, k, g, beta, scratch, q_start, q_len, S, H, G, dim);
+    chunk_prep_kernel<DP, MODE><<<dim3(slots, H), 128, smem1, st>>>(q, k, g, beta, scratch, q_start, q_len, S, H, G, dim, shortest);
     MB_LAUNCH_CHECK();
     const dim3 grid((vdim + LC_COLS - 1) / LC_COLS, H, S);
     chunk_walk_kernel<DP, MODE, TRANS><<<grid, 256, smem2, st>>>(v, o, state, state_stride, scratch, q_start, q_len, state_slot, H,
-                                                                 dim, vdim, err);
+                                                                 dim, vdim, shortest, err);
     MB_LAUNCH_CHECK();
     return 0;
 }
@@ -542,22 +543,23 @@ MB_API int mb_linear_chunks_record(int dim, int vdim, int mode) {
 }
 
 // q, k (N, G, dim), v, o (N, H, vdim), all of them and g on 16-byte boundaries; state: a head's matrix at h dim vdim,
-// (dim, vdim), with mode 4 (vdim, dim).  scratch: (N / 32 + min(S, N / 32)) H records.  Sequences of fewer than 32 tokens are left as they are.
+// (dim, vdim), with mode 4 (vdim, dim).  scratch: (N / 32 + min(S, N / shortest)) H records.  Sequences of fewer than
+// `shortest` tokens (32 or more) are left as they are.
 MB_API int mb_linear_chunks(const float* q, const float* k, const float* v, const float* g, const float* beta, float* o,
                             float* state, long long state_stride, const int* q_start, const int* q_len,
-                            const int* state_slot, int S, int N, int H, int G, int dim, int vdim, int mode, float* scratch,
+                            const int* state_slot, int S, int N, int H, int G, int dim, int vdim, int mode, int shortest, float* scratch,
                             long long scratch_floats, int* err, cudaStream_t st) {
     if (S == 0 || N == 0) return 0;
-    if (G < 1 || H % G || H > 65535 || S > 65535 || !mb_linear_chunks_record(dim, vdim, mode)) return -2;
+    if (G < 1 || H % G || H > 65535 || S > 65535 || shortest < LC_MIN || !mb_linear_chunks_record(dim, vdim, mode)) return -2;
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o | (uintptr_t)scratch) & 15) return -2;
     if ((mode == 0 || mode == 1 || mode == 3) && ((uintptr_t)g & 15)) return -2;
     if ((mode == 0 || mode == 3) && !beta) return -2;
 #define LC_CASE(MODE)                                                                                                       \
     if (mode == MODE)                                                                                                       \
         return dim <= 64 ? lc_launch<64, MODE>(q, k, v, g, beta, o, state, state_stride, q_start, q_len, state_slot, S, N, H, G, \
-                                               dim, vdim, scratch, scratch_floats, err, st)                                 \
+                                               dim, vdim, shortest, scratch, scratch_floats, err, st)                                 \
                          : lc_launch<128, MODE>(q, k, v, g, beta, o, state, state_stride, q_start, q_len, state_slot, S, N, H, \
-                                                G, dim, vdim, scratch, scratch_floats, err, st);
+                                                G, dim, vdim, shortest, scratch, scratch_floats, err, st);
     LC_CASE(0) LC_CASE(1) LC_CASE(2) LC_CASE(3) LC_CASE(4)
 #undef LC_CASE
     return -2;

@@ -1609,11 +1609,9 @@ def gated_scan(q, k, v, g, o, state, seq, H, G, dim, vdim, per_head, bonus=None,
              dim, vdim, 1 if per_head else 0, 1 if q.shape[0] > 4 * S and not below else 0, int(below), _stream()), "gated_scan")
 
 
-# ---- the linear-attention recurrences over long stretches, 32 tokens at a time (linear_chunks.cu).  A step runs them when it
-# has more than `tokens` tokens beyond one a sequence.  One sequence, 16 heads of 128 x 128, delta rule, chunks / scan: 65
-# tokens 34 / 28 us, 128 36 / 47, 512 75 / 168, 2,048 228 / 646.  Sequences of fewer than `shortest` tokens stay with the
-# scans, which then follow the chunks' kernels.
-CHUNKS = {"tokens": 80, "shortest": 32}
+# ---- the linear-attention recurrences over long stretches, 32 tokens at a time (linear_chunks.cu): the sequences of a step
+# that have at least `shortest` tokens, where the step has one (linear_chunks_shortest).
+CHUNKS = {"tokens": 80, "delta": (80, 160), "channels": (64, 64), "heads": (80, 80), "wkv": (64, 64), "fixed": (64, 96)}
 CHUNK_MODES = {"delta": 0, "channels": 1, "heads": 2, "wkv": 3, "fixed": 4}
 
 
@@ -1624,14 +1622,41 @@ def _chunk_record(dim, vdim, mode):
 
 
 def linear_chunks_supports(N, S, dim, vdim, mode):
-    """whether a step of N tokens in S sequences runs the chunk form: by lengths alone, as a captured step demands"""
+    """whether a step of N tokens in S sequences may run the chunk form: the sizes fit and it has more than `tokens` tokens
+    beyond one a sequence"""
     return N - S > CHUNKS["tokens"] and 4 <= dim <= 128 and dim % 4 == 0 and vdim >= 4 and vdim % 4 == 0
 
 
-def linear_chunks_slots(N, S):
+def linear_chunks_shortest(lengths, H, dim, vdim, mode):
+    """From how many tokens on the sequences of a step (their lengths, on the host) go through the chunk form; 0: none does.
+    A record costs its 32 tokens whatever it holds, and what is shorter takes a scan of its own after the chunks.  Measured, us,
+    chunks / scan (16 heads of 128 x 128; 24 by channel, 48 of 128 x 64 by head):
+      one sequence      of 65 tokens  delta 30/29  channels 26/27  heads 28/27  wkv 24/25;  82: 30/33  28/33  28/31  24/29, fixed 23/36
+      16 of them        of 33 tokens  delta 157/90  heads 140/137  fixed 87/59;  48: 156/123  142/170  91/78;  65: 203/160  183/221
+                        112/101;  96: 208/227  191/301  116/141
+      four of 128       delta 89/84, of 160: 89/104 (more blocks than SMs, each an SM's shared memory: from 160 tokens on)
+      100 beside ten of 20 tokens     delta 75/61  heads 77/84  fixed 58/45
+      128 beside 37 decoded tokens    delta 75/74  channels 91/133  fixed, 32 heads, 75/61;  200 beside 16: delta 60/94  fixed 50/66
+      500 beside sixteen of 60        delta, 24 heads, 323/291  channels 243/338
+    (the scan of the short sequences alone runs the layout for short stretches, which is what channels, heads and wkv gain by)"""
+    if not linear_chunks_supports(sum(lengths), len(lengths), dim, vdim, mode):
+        return 0
+    one, more = CHUNKS[mode]
+    shortest = one if sum(n >= one for n in lengths) * H * -(-vdim // 16) <= 148 else more
+    longest, rest = max(lengths), [n for n in lengths if n < shortest]
+    if longest < shortest:
+        return 0
+    if rest and mode in ("delta", "fixed"):
+        pays = longest >= 100 + 3 * len(rest) and 2 * sum(rest) <= 3 * (sum(lengths) - sum(rest))
+    else:
+        pays = not rest or longest >= 128
+    return shortest if pays else 0
+
+
+def linear_chunks_slots(N, S, shortest=32):
     """the most chunks that N tokens in S sequences make: an upper bound of the sum of ceil(length / 32) over the sequences of at
-    least 32 tokens, of which there are at most N / 32"""
-    return N // 32 + min(S, N // 32)
+    least `shortest` tokens, of which there are at most N / shortest"""
+    return N // 32 + min(S, N // shortest)
 
 
 def linear_chunks_floats(H, dim, vdim, mode):
@@ -1639,33 +1664,35 @@ def linear_chunks_floats(H, dim, vdim, mode):
     return H * _chunk_record(dim, vdim, mode)
 
 
-def linear_chunks(mode, q, k, v, g, o, state, seq, H, G, dim, vdim, beta=None, scratch=None):
+def linear_chunks(mode, q, k, v, g, o, state, seq, H, G, dim, vdim, beta=None, scratch=None, shortest=32, rest=None):
     """The recurrence of delta_rule ("delta", beta (N, H)), gated_scan ("channels"; "heads": per_head; "wkv": beta = its
     bonus) or retention ("fixed", g = its decay, state (vdim, dim) a head) over the same arguments, 32 tokens at a time.
-    dim up to 128, dim and vdim multiples of 4; sequences of fewer than 32 tokens go through the token-by-token kernels
-    here.  scratch (linear_chunks_slots(N, S), linear_chunks_floats(..)) float32 (made
-    here when absent)."""
+    dim up to 128, dim and vdim multiples of 4; sequences of fewer than `shortest` tokens (32 or more) go through the
+    token-by-token kernels after it.  scratch: linear_chunks_slots(N, S, shortest) * linear_chunks_floats(..) float32 (made
+    here when absent).  rest: whether the step has such sequences (None: not known)."""
     _cuda(q, k, v, g, o, state, beta, *seq)
     N, S = q.shape[0], seq[0].numel()
     if not _chunk_record(dim, vdim, mode):
         raise KernelError("linear_chunks: the kernel does not take these sizes")
     if scratch is None:
-        scratch = torch.empty(linear_chunks_slots(N, S), linear_chunks_floats(H, dim, vdim, mode), dtype=torch.float32,
-                              device=q.device)
+        scratch = torch.empty(linear_chunks_slots(N, S, shortest) * linear_chunks_floats(H, dim, vdim, mode),
+                              dtype=torch.float32, device=q.device)
     f = _fn("linear_chunks", "mb_linear_chunks",
-            [c_void_p] * 7 + [c_ll] + [c_void_p] * 3 + [c_int] * 7 + [c_void_p, c_ll, c_void_p, c_void_p])
+            [c_void_p] * 7 + [c_ll] + [c_void_p] * 3 + [c_int] * 8 + [c_void_p, c_ll, c_void_p, c_void_p])
     _check(f(_p(q), _p(k), _p(v), _p(g), _p(beta), _p(o), _p(state), state.stride(0), *[_p(t) for t in seq], S, N, H, G, dim,
-             vdim, CHUNK_MODES[mode], _p(scratch), scratch.numel(), _p(error_word(q.device)), _stream()), "linear_chunks")
+             vdim, CHUNK_MODES[mode], int(shortest), _p(scratch), scratch.numel(), _p(error_word(q.device)), _stream()),
+           "linear_chunks")
     COUNTERS["launches"] += 1           # the chunks' own part, and the walk along them
-    short = CHUNKS["shortest"]
-    if S == 1 and N >= short:
+    if rest is None:
+        rest = S > 1 or N < shortest
+    if not rest:
         return
     if mode == "delta":
-        delta_rule(q, k, v, g, beta, o, state, seq, H, G, dim, vdim, below=short)
+        delta_rule(q, k, v, g, beta, o, state, seq, H, G, dim, vdim, below=shortest)
     elif mode == "fixed":
-        retention(q, k, v, g, o, state, seq, H, dim, vdim, below=short)
+        retention(q, k, v, g, o, state, seq, H, dim, vdim, below=shortest)
     else:
-        gated_scan(q, k, v, g, o, state, seq, H, G, dim, vdim, mode == "heads", bonus=beta, below=short)
+        gated_scan(q, k, v, g, o, state, seq, H, G, dim, vdim, mode == "heads", bonus=beta, below=shortest)
 
 
 def token_mix(h, mu, state, seq, out):

@@ -276,17 +276,32 @@ class StepContext:
         return h
 
 
+def plan_chunks(ctx, mode, H, dim, vdim):
+    """Host side, once per step and kind of recurrence: from how many tokens on the step's sequences go through the chunk form
+    (ops.linear_chunks), and whether shorter ones are left for the scan.  Both are part of a captured step's shape, as the length
+    of an array.  Not on the float32 path: there a prompt's sums run in the same order however it is cut into steps."""
+    import torch
+    key = ("chunks", mode, H, dim, vdim)
+    if key in ctx.memo:
+        return
+    shortest = 0 if ctx.dtype != torch.bfloat16 else ctx.ops.linear_chunks_shortest(ctx.q_len, H, dim, vdim, mode)
+    rest = shortest > 0 and min(ctx.q_len) < shortest
+    ctx.memo[key] = (shortest, rest)
+    code = 1 + 2 * ctx.ops.CHUNKS[mode].index(shortest) + rest if shortest else 0
+    ctx.inputs.add("_".join(map(str, key)), [0] * code)
+
+
 def chunked_recurrence(ctx, mode, q, k, v, g, o, state, H, G, dim, vdim, beta=None):
-    """Runs a linear-attention recurrence in its chunk form (ops.linear_chunks) when the step has long stretches.  -> whether
-    it did.  Not on the float32 path: there a prompt's sums run in the same order however it is cut into steps.  The scratch is
-    one buffer for all layers of these sizes, reserved for the largest step of up to 64 sequences, so that it hardly ever grows
-    (a growth makes captured steps stale)."""
+    """Runs a linear-attention recurrence in its chunk form where plan_chunks found long stretches.  -> whether it did.  The
+    scratch is one buffer for all layers of these sizes, reserved for the largest step of up to 64 sequences, so that it hardly
+    ever grows (a growth makes captured steps stale)."""
     import torch
     ops, N, S = ctx.ops, ctx.N, ctx.S
-    if ctx.dtype != torch.bfloat16 or not ops.linear_chunks_supports(N, S, dim, vdim, mode):
+    shortest, rest = ctx.memo.get(("chunks", mode, H, dim, vdim), (0, False))
+    if not shortest:
         return False
-    scratch = ctx.ws.get("linear_chunks", ops.linear_chunks_slots(N, S), (ops.linear_chunks_floats(H, dim, vdim, mode),),
-                         torch.float32, reserve=ops.linear_chunks_slots(ctx.ws.max_rows, max(S, 64)))
+    scratch = ctx.ws.get("linear_chunks", ops.linear_chunks_slots(N, S, shortest), (ops.linear_chunks_floats(H, dim, vdim, mode),),
+                         torch.float32, reserve=ops.linear_chunks_slots(ctx.ws.max_rows, max(S, 64), min(ops.CHUNKS[mode])))
     ops.linear_chunks(mode, q, k, v, g, o, state, (ctx.dev("q_start"), ctx.dev("q_len"), ctx.dev("state_slot")), H, G, dim, vdim,
-                      beta=beta, scratch=scratch)
+                      beta=beta, scratch=scratch, shortest=shortest, rest=rest)
     return True

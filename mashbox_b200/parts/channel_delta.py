@@ -22,7 +22,7 @@ logarithms, softplus, beta, the unit norms, the state and the recurrence are flo
 from ..cache.manager import StateNeed
 from ..errors import ConfigError
 from ..weights.loader import Want
-from .base import chunked_recurrence, register
+from .base import chunked_recurrence, plan_chunks, register
 from .conv import plan_sequences, state_view, step_sequences
 
 
@@ -94,6 +94,7 @@ class ChannelDelta:
 
     def prepare(self, ctx):
         plan_sequences(ctx)
+        plan_chunks(ctx, "delta", self.H, self.dim, self.vdim)
 
     def forward(self, ctx, h, run):
         import torch

@@ -15,7 +15,7 @@ state, the recurrence and the norm are float32.
 """
 from ..cache.manager import StateNeed
 from ..weights.loader import Want
-from .base import chunked_recurrence, register
+from .base import chunked_recurrence, plan_chunks, register
 
 
 class GatedLinearAttention:
@@ -60,7 +60,7 @@ class GatedLinearAttention:
         return StateNeed((self.state_floats(),), "float32")
 
     def prepare(self, ctx):
-        pass
+        plan_chunks(ctx, "channels", self.H, self.dim, self.vdim)
 
     def forward(self, ctx, h, run, out="delta"):
         import torch

@@ -16,7 +16,7 @@ the output product.  Angles, the state, the recurrence and the norm are float32.
 from ..cache.manager import StateNeed
 from ..errors import ConfigError
 from ..weights.loader import Want
-from .base import PartSpec, chunked_recurrence, make, register
+from .base import PartSpec, chunked_recurrence, make, plan_chunks, register
 
 
 class Retention:
@@ -67,7 +67,7 @@ class Retention:
         return StateNeed((self.state_floats(),), "float32")
 
     def prepare(self, ctx):
-        pass
+        plan_chunks(ctx, "fixed", self.H, self.dim, self.vdim)
 
     def prepare_rows(self, ctx, rows, q, k, v):
         """q, k, v in float32 from the rows of the product"""

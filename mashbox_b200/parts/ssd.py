@@ -19,7 +19,7 @@ and the norm are float32.
 from ..cache.manager import StateNeed
 from ..errors import ConfigError
 from ..weights.loader import Want
-from .base import chunked_recurrence, register
+from .base import chunked_recurrence, plan_chunks, register
 from .conv import plan_sequences, state_view, step_sequences
 
 
@@ -72,6 +72,7 @@ class StateSpaceDuality:
 
     def prepare(self, ctx):
         plan_sequences(ctx)
+        plan_chunks(ctx, "heads", self.H, self.NS, self.P)
 
     def forward(self, ctx, h, run, out="delta"):
         import torch

@@ -19,7 +19,7 @@ and the norm are float32 arithmetic.
 from ..cache.manager import StateNeed
 from ..errors import ConfigError
 from ..weights.loader import Want
-from .base import chunked_recurrence, register
+from .base import chunked_recurrence, plan_chunks, register
 from .conv import plan_sequences, step_sequences
 
 STREAMS = ("r", "k", "v", "g", "w")
@@ -70,6 +70,7 @@ class WkvMixing:
 
     def prepare(self, ctx):
         plan_sequences(ctx)
+        plan_chunks(ctx, "wkv", self.H, self.dim, self.dim)
 
     def forward(self, ctx, h, run, out="delta"):
         import torch

@@ -158,6 +158,42 @@ def test_many_sequences_side_by_side(kind, lens):
     ops.check_error_word(ops.error_word(DEV))
 
 
+@pytest.mark.parametrize("shortest", (32, 64, 160))
+@pytest.mark.parametrize("kind", KINDS)
+def test_sequences_below_the_shortest_are_the_scans(kind, shortest):
+    """lengths on both sides of the line; those below it get the bits of the scan over them alone, and without `rest` are left
+    as they are"""
+    from mashbox_b200 import ops
+    H, dim, vdim, lens = 2, 64, 32, [31, 32, 63, 64, 159, 160, 161, 1, 300]
+    N = sum(lens)
+    q, k, v, z, beta = inputs(kind, shortest, N, H, H, dim, vdim, "slow")
+    dev = lambda x: x.reshape(x.shape[0], -1).contiguous().to(DEV)
+    g = z.reshape(-1).contiguous().to(DEV) if kind == "fixed" else dev(z)
+    start = torch.randn(len(lens), H * dim * vdim, generator=torch.Generator().manual_seed(1)) * 0.1
+    seq = (i32(np.concatenate([[0], np.cumsum(lens)[:-1]])), i32(lens), i32(list(range(len(lens)))))
+    outs = []
+    for form in ("scan", "chunks", "no rest"):
+        o, state = torch.full((N, H * vdim), 7.0, device=DEV), start.to(DEV)
+        if form == "scan":
+            launch(ops, kind, False, q, k, v, z, beta, o, state, seq, H, H, dim, vdim)
+        else:
+            ops.linear_chunks(kind, dev(q), dev(k), dev(v), g, o, state, seq, H, H, dim, vdim,
+                              beta=dev(beta) if kind in ("delta", "wkv") else None, shortest=shortest,
+                              rest=None if form == "chunks" else False)
+        outs.append((o, state))
+    (so, ss), (co, cs), (no, ns) = outs
+    lo = 0
+    for s, n in enumerate(lens):
+        rows, short = slice(lo, lo + n), n < shortest
+        for a, b in ((so[rows], co[rows]), (ss[s], cs[s])):
+            assert float((a - b).norm() / a.norm()) < 1e-6         # float32 sums in another order
+        assert bool((no[rows] == 7.0).all()) == short and torch.equal(ns[s].cpu(), start[s]) == short
+        if not short:
+            assert torch.equal(no[rows], co[rows]) and torch.equal(ns[s], cs[s])
+        lo += n
+    ops.check_error_word(ops.error_word(DEV))
+
+
 @pytest.mark.parametrize("kind", ("channels", "heads", "wkv"))
 def test_decoded_tokens_beside_a_prompt_run_as_without_it(kind):
     """the scan of the short sequences lays the state out as it does in a step of theirs alone: the same bits"""
