@@ -293,15 +293,16 @@ def plan_chunks(ctx, mode, H, dim, vdim):
 
 def chunked_recurrence(ctx, mode, q, k, v, g, o, state, H, G, dim, vdim, beta=None):
     """Runs a linear-attention recurrence in its chunk form where plan_chunks found long stretches.  -> whether it did.  The
-    scratch is one buffer for all layers of these sizes, reserved for the largest step of up to 64 sequences, so that it hardly
-    ever grows (a growth makes captured steps stale)."""
+    scratch is one flat buffer for all layers of a model, asked for at the size of the largest step of up to 64 sequences, so
+    that it hardly ever grows once every layer has run (a growth makes captured steps stale)."""
     import torch
-    ops, N, S = ctx.ops, ctx.N, ctx.S
+    ops = ctx.ops
     shortest, rest = ctx.memo.get(("chunks", mode, H, dim, vdim), (0, False))
     if not shortest:
         return False
-    scratch = ctx.ws.get("linear_chunks", ops.linear_chunks_slots(N, S, shortest), (ops.linear_chunks_floats(H, dim, vdim, mode),),
-                         torch.float32, reserve=ops.linear_chunks_slots(ctx.ws.max_rows, max(S, 64), min(ops.CHUNKS[mode])))
+    most = max(ctx.N, ctx.ws.max_rows)
+    floats = ops.linear_chunks_slots(most, max(ctx.S, 64), min(ops.CHUNKS[mode])) * ops.linear_chunks_floats(H, dim, vdim, mode)
+    scratch = ctx.ws.get("linear_chunks", floats, (), torch.float32, reserve=floats)
     ops.linear_chunks(mode, q, k, v, g, o, state, (ctx.dev("q_start"), ctx.dev("q_len"), ctx.dev("state_slot")), H, G, dim, vdim,
                       beta=beta, scratch=scratch, shortest=shortest, rest=rest)
     return True

@@ -70,3 +70,19 @@ def test_the_decision_is_part_of_a_captured_steps_shape():
     assert not chunked_recurrence(ctx, "delta", *[None] * 6, 16, 16, 128, 128) and not calls
     assert all(len(a) == 0 for a in ctx.inputs.arrays.values())
 
+
+def test_one_scratch_for_all_layers():
+    """two kinds of layers share one buffer, which the largest step does not make grow"""
+    ctx, calls = context([300, 200])
+    for mode, H in (("channels", 24), ("heads", 48)):
+        plan_chunks(ctx, mode, H, 128, 64)
+        assert chunked_recurrence(ctx, mode, *[None] * 6, H, H, 128, 64)
+    assert len(ctx.ws.buffers) == 1
+    made = ctx.ws.generation
+    for lengths in ([64] * 33, [2112], [80] * 26, [500] * 4 + [1] * 112):
+        step, _ = context(lengths)
+        step.ws = ctx.ws
+        for mode, H in (("channels", 24), ("heads", 48)):
+            plan_chunks(step, mode, H, 128, 64)
+            assert chunked_recurrence(step, mode, *[None] * 6, H, H, 128, 64) or max(lengths) < 80
+    assert ctx.ws.generation == made and len(ctx.ws.buffers) == 1
