@@ -205,35 +205,44 @@ __global__ void moe_experts_down_kernel(const float* __restrict__ act, const int
     }
 }
 
-// The same two kernels for steps of few pairs (up to MOE_FEW), where tokens share experts: the block of the first pair that
-// chose an expert works for all pairs that did, the blocks of the others leave, so that an expert's matrices come from
-// memory once.  (A step of 8 tokens that choose 8 of 64 experts each, D 4,096, F 2,048: some 40 experts of 50 MB are read
-// for 64 pairs.)  What bounds it is that read: a block asks the L2 for all of its rows before it brings the inputs in, a warp
-// then has two rows of 16 bytes a lane and MOE_AHEAD of each under way, and up to MOE_TOKENS inputs in shared memory meet a
-// weight while it is in registers.  Every dot product runs in the order of lane_dot.  Measured on that step, a block per
-// pair / per expert: gate and up 337 / 222 us (6.0 TB/s), down 171 / 123 us (5.4 TB/s).
+// The same two kernels for steps of few pairs (up to MOE_FEW), where tokens share experts: the pairs of an expert are taken
+// together, MOE_TOKENS of them a block, so that an expert with up to MOE_TOKENS pairs comes from memory once (a step of 8
+// tokens that choose 8 of 64 experts each, D 4,096, F 2,048: some 40 experts of 50 MB are read for 64 pairs), and one with
+// more meets its further groups in other blocks at about the same time, so that they find it in the L2.  What bounds them is
+// that read: a block asks the L2 for all of its rows before it brings the inputs in, a warp then has two rows of 16 bytes a
+// lane and MOE_AHEAD of each under way, and the inputs in shared memory meet a weight while it is in registers.  Every dot
+// product runs in the order of lane_dot.  A block has 8 rows of gate and of up (of down four times as many) up to 64 pairs,
+// 16 beyond: with few blocks the last, partly filled round of them weighs more than the inputs brought in twice as often.
+// Measured, both kernels, us, a block per pair / now: D 4,096, F 2,048, 8 of 64 experts: one token 100 / 91, two 183 / 144,
+// four 290 / 232, eight 509 / 334 (5.9 TB/s), sixteen 968 / 499, sixteen that share favourites 963 / 476 (588 with one block
+// an expert); D 2,048, F 1,408, 6 of 64: 54 / 36, 63 / 52, 110 / 85, 161 / 126, 280 / 182, 278 / 167; D 2,048, F 768, 8 of
+// 128: 46 / 32, 56 / 46, 75 / 69, 124 / 108, 218 / 159, 212 / 144.  (Plain loads instead of __ldcs: 2 to 10 % slower.)
 #define MOE_FEW 512
 #define MOE_TOKENS 4
 #define MOE_AHEAD 4
-#define MOE_FEW_ROWS 16        // rows of gate and of up a block; of down four times as many
 
-// the pairs of this block's expert, in order, into list -> their number; 0 for every block but the first pair's
+// The pairs of an expert, in order, in groups of MOE_TOKENS: the block of a group's first pair gets the group into list -> their
+// number; 0 for the blocks of the other pairs.
 __device__ __forceinline__ int moe_sharers(const int* __restrict__ ids, int pair, int P, int E, int& e, int* list, int* count) {
     auto expert = [&](int p) { const int x = ids[p]; return x < 0 || x >= E ? 0 : x; };
     e = expert(pair);
     int earlier = 0;
-    for (int p = threadIdx.x; p < pair; p += blockDim.x) earlier |= expert(p) == e;
-    if (__syncthreads_or(earlier)) return 0;
+    for (int p0 = 0; p0 < pair; p0 += blockDim.x) {
+        const int p = p0 + threadIdx.x;
+        earlier += __syncthreads_count(p < pair && expert(p) == e);
+    }
+    if (earlier % MOE_TOKENS) return 0;
     if (threadIdx.x < 32) {
         int n = 0;
-        for (int p0 = pair; p0 < P; p0 += 32) {
+        for (int p0 = pair; p0 < P && n < MOE_TOKENS; p0 += 32) {
             const int p = p0 + threadIdx.x;
             const bool mine = p < P && expert(p) == e;
             const unsigned who = __ballot_sync(0xffffffffu, mine);
-            if (mine) list[n + __popc(who & ((1u << threadIdx.x) - 1))] = p;
+            const int at = n + __popc(who & ((1u << threadIdx.x) - 1));
+            if (mine && at < MOE_TOKENS) list[at] = p;
             n += __popc(who);
         }
-        if (threadIdx.x == 0) *count = n;
+        if (threadIdx.x == 0) *count = min(n, MOE_TOKENS);
     }
     __syncthreads();
     return *count;
@@ -310,76 +319,70 @@ __device__ __forceinline__ void moe_two_rows(const bf16* __restrict__ w0, const 
         }
 }
 
-// grid (pairs, stretches of MOE_FEW_ROWS rows of F), 256 threads; dynamic shared: MOE_TOKENS rows of D
+// grid (pairs, stretches of ROWS rows of F), 256 threads; dynamic shared: MOE_TOKENS rows of D
+template <int ROWS>
 __global__ void __launch_bounds__(256, 3)
 moe_few_up_kernel(const bf16* __restrict__ h, const int* __restrict__ ids, const bf16* __restrict__ wg,
                   const bf16* __restrict__ wu, long long gu_stride, float* __restrict__ act, int P, int D, int F, int E, int top,
                   float limit, float alpha, float shift, const float* __restrict__ in_wts) {
     extern __shared__ __align__(16) unsigned char few_smem[];
-    __shared__ int list[MOE_FEW], count;
+    __shared__ int list[MOE_TOKENS], count;
     bf16* hx = reinterpret_cast<bf16*>(few_smem);
     int e;
-    const int sharers = moe_sharers(ids, blockIdx.x, P, E, e, list, &count);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j0 = blockIdx.y * MOE_FEW_ROWS;
+    const int n = moe_sharers(ids, blockIdx.x, P, E, e, list, &count);
+    if (n == 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j0 = blockIdx.y * ROWS;
     const bf16 *g_rows = wg + (size_t)e * gu_stride, *u_rows = wu + (size_t)e * gu_stride;
-    if (sharers && threadIdx.x < 2)
-        moe_ask((threadIdx.x ? u_rows : g_rows) + (size_t)j0 * D, min(F - j0, MOE_FEW_ROWS), D);
-    for (int at = 0; at < sharers; at += MOE_TOKENS) {
-        const int n = min(MOE_TOKENS, sharers - at);
-        if (at) __syncthreads();
-        for (int idx = threadIdx.x; idx < n * (D / 8); idx += blockDim.x) {
-            const int t = idx / (D / 8), i = idx - t * (D / 8);
-            reinterpret_cast<uint4*>(hx + (size_t)t * D)[i] =
-                reinterpret_cast<const uint4*>(h + (size_t)(list[at + t] / top) * D)[i];
-        }
-        __syncthreads();
-        for (int j = j0 + warp; j < min(F, j0 + MOE_FEW_ROWS); j += 8) {
-            float g[MOE_TOKENS], u[MOE_TOKENS];
-            moe_two_rows(g_rows + (size_t)j * D, u_rows + (size_t)j * D, hx, D, D, n, lane, g, u);
+    if (threadIdx.x < 2) moe_ask((threadIdx.x ? u_rows : g_rows) + (size_t)j0 * D, min(F - j0, ROWS), D);
+    for (int idx = threadIdx.x; idx < n * (D / 8); idx += blockDim.x) {
+        const int t = idx / (D / 8), i = idx - t * (D / 8);
+        reinterpret_cast<uint4*>(hx + (size_t)t * D)[i] = reinterpret_cast<const uint4*>(h + (size_t)(list[t] / top) * D)[i];
+    }
+    __syncthreads();
+    for (int j = j0 + warp; j < min(F, j0 + ROWS); j += 8) {
+        float g[MOE_TOKENS], u[MOE_TOKENS];
+        moe_two_rows(g_rows + (size_t)j * D, u_rows + (size_t)j * D, hx, D, D, n, lane, g, u);
 #pragma unroll
-            for (int t = 0; t < MOE_TOKENS; t++)
-                if (t < n && lane == t) {
-                    const int pair = list[at + t];
-                    const float rs = in_wts ? in_wts[pair] : 1.0f;
-                    const float gg = fminf(g[t] * rs, limit), uu = fminf(fmaxf(u[t] * rs, -limit), limit);
-                    act[(size_t)pair * F + j] = gg / (1.0f + expf(-alpha * gg)) * (uu + shift);
-                }
-        }
+        for (int t = 0; t < MOE_TOKENS; t++)
+            if (t < n && lane == t) {
+                const int pair = list[t];
+                const float rs = in_wts ? in_wts[pair] : 1.0f;
+                const float gg = fminf(g[t] * rs, limit), uu = fminf(fmaxf(u[t] * rs, -limit), limit);
+                act[(size_t)pair * F + j] = gg / (1.0f + expf(-alpha * gg)) * (uu + shift);
+            }
     }
 }
 
-// grid (pairs, stretches of 4 MOE_FEW_ROWS rows of D), 256 threads; dynamic shared: MOE_TOKENS rows of F floats
+// grid (pairs, stretches of 4 ROWS rows of D), 256 threads; dynamic shared: MOE_TOKENS rows of F floats
+template <int ROWS>
 __global__ void __launch_bounds__(256, 3)
 moe_few_down_kernel(const float* __restrict__ act, const int* __restrict__ ids, const bf16* __restrict__ wd,
                     float* __restrict__ y, int P, int D, int F, int E) {
     extern __shared__ __align__(16) unsigned char few_smem[];
-    __shared__ int list[MOE_FEW], count;
+    __shared__ int list[MOE_TOKENS], count;
     float* ax = reinterpret_cast<float*>(few_smem);
     int e;
-    const int sharers = moe_sharers(ids, blockIdx.x, P, E, e, list, &count);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d0 = blockIdx.y * 4 * MOE_FEW_ROWS;
+    const int n = moe_sharers(ids, blockIdx.x, P, E, e, list, &count);
+    if (n == 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d0 = blockIdx.y * 4 * ROWS;
     const bf16* rows = wd + (size_t)e * D * F;
-    if (sharers && threadIdx.x == 0) moe_ask(rows + (size_t)d0 * F, min(D - d0, 4 * MOE_FEW_ROWS), F);
-    for (int at = 0; at < sharers; at += MOE_TOKENS) {
-        const int n = min(MOE_TOKENS, sharers - at);
-        if (at) __syncthreads();
-        for (int idx = threadIdx.x; idx < n * (F / 4); idx += blockDim.x) {
-            const int t = idx / (F / 4), j = (idx - t * (F / 4)) * 4;
-            *reinterpret_cast<float4*>(ax + (size_t)t * F + moe_place(j, F)) =
-                *reinterpret_cast<const float4*>(act + (size_t)list[at + t] * F + j);
-        }
-        __syncthreads();
-        for (int d = d0 + 2 * warp; d < min(D, d0 + 4 * MOE_FEW_ROWS); d += 16) {        // D is even: rows d and d + 1
-            float a[MOE_TOKENS], b[MOE_TOKENS];
-            moe_two_rows(rows + (size_t)d * F, rows + (size_t)(d + 1) * F, ax, F, F, n, lane, a, b);
+    if (threadIdx.x == 0) moe_ask(rows + (size_t)d0 * F, min(D - d0, 4 * ROWS), F);
+    for (int idx = threadIdx.x; idx < n * (F / 4); idx += blockDim.x) {
+        const int t = idx / (F / 4), j = (idx - t * (F / 4)) * 4;
+        *reinterpret_cast<float4*>(ax + (size_t)t * F + moe_place(j, F)) =
+            *reinterpret_cast<const float4*>(act + (size_t)list[t] * F + j);
+    }
+    __syncthreads();
+    for (int d = d0 + 2 * warp; d < min(D, d0 + 4 * ROWS); d += 16) {        // D is even: rows d and d + 1
+        float a[MOE_TOKENS], b[MOE_TOKENS];
+        moe_two_rows(rows + (size_t)d * F, rows + (size_t)(d + 1) * F, ax, F, F, n, lane, a, b);
 #pragma unroll
-            for (int t = 0; t < MOE_TOKENS; t++)
-                if (t < n && lane == t) {
-                    float* dst = y + (size_t)list[at + t] * D + d;
-                    dst[0] = a[t];
-                    dst[1] = b[t];
-                }
-        }
+        for (int t = 0; t < MOE_TOKENS; t++)
+            if (t < n && lane == t) {
+                float* dst = y + (size_t)list[t] * D + d;
+                dst[0] = a[t];
+                dst[1] = b[t];
+            }
     }
 }
 
@@ -436,31 +439,37 @@ MB_API int mb_moe_experts_f32(const void* h, const int* ids, const void* wg, con
                                      act, N, D, F, E, top, limit, alpha, shift, in_wts, st);
 }
 
+template <int ROWS>
+static int moe_few_launch(const bf16* h, const int* ids, const bf16* wg, const bf16* wu, long long gu_stride, const bf16* wd,
+                          float* y, float* act, int P, int D, int F, int E, int top, float limit, float alpha, float shift,
+                          const float* in_wts, cudaStream_t st) {
+    static bool configured = false;
+    if (!configured) {
+        const auto most = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        cudaError_t e = cudaFuncSetAttribute(moe_few_up_kernel<ROWS>, most, MOE_TOKENS * 12000 * 2);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_few_down_kernel<ROWS>, most, MOE_TOKENS * 12000 * 4);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    moe_few_up_kernel<ROWS><<<dim3(P, (F + ROWS - 1) / ROWS), 256, (size_t)MOE_TOKENS * D * 2, st>>>(
+        h, ids, wg, wu, gu_stride, act, P, D, F, E, top, limit, alpha, shift, in_wts);
+    MB_LAUNCH_CHECK();
+    moe_few_down_kernel<ROWS><<<dim3(P, (D + 4 * ROWS - 1) / (4 * ROWS)), 256, (size_t)MOE_TOKENS * F * 4, st>>>(
+        act, ids, wd, y, P, D, F, E);
+    MB_LAUNCH_CHECK();
+    return 0;
+}
+
 MB_API int mb_moe_experts_bf16(const void* h, const int* ids, const void* wg, const void* wu, long long gu_stride,
                                const void* wd, float* y, float* act, int N, int D, int F, int E, int top, float limit,
                                float alpha, float shift, const float* in_wts, cudaStream_t st) {
-    // one read of an expert for all its pairs: the rows must allow 16-byte loads, the inputs must fit shared memory
+    // the rows must allow 16-byte loads, the inputs must fit shared memory
     const uintptr_t ptrs = (uintptr_t)h | (uintptr_t)wg | (uintptr_t)wu | (uintptr_t)wd | (uintptr_t)act;
     if (N > 0 && top > 0 && (long long)N * top <= MOE_FEW && D > 0 && F > 0 && D % 8 == 0 && F % 8 == 0 && gu_stride % 8 == 0 &&
-        D <= 12000 && F <= 12000 && (ptrs & 15) == 0) {
-        const size_t up = (size_t)MOE_TOKENS * D * 2, down = (size_t)MOE_TOKENS * F * 4;
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t e = cudaFuncSetAttribute(moe_few_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_TOKENS * 12000 * 2);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(moe_few_down_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_TOKENS * 12000 * 4);
-            if (e != cudaSuccess) return (int)e;
-            configured = true;
-        }
-        const int P = N * top;
-        moe_few_up_kernel<<<dim3(P, (F + MOE_FEW_ROWS - 1) / MOE_FEW_ROWS), 256, up, st>>>(
-            (const bf16*)h, ids, (const bf16*)wg, (const bf16*)wu, gu_stride, act, P, D, F, E, top, limit, alpha, shift, in_wts);
-        MB_LAUNCH_CHECK();
-        moe_few_down_kernel<<<dim3(P, (D + 4 * MOE_FEW_ROWS - 1) / (4 * MOE_FEW_ROWS)), 256, down, st>>>(act, ids, (const bf16*)wd, y,
-                                                                                                        P, D, F, E);
-        MB_LAUNCH_CHECK();
-        return 0;
-    }
+        D <= 12000 && F <= 12000 && (ptrs & 15) == 0)
+        return (N * top <= 64 ? moe_few_launch<8> : moe_few_launch<16>)(
+            (const bf16*)h, ids, (const bf16*)wg, (const bf16*)wu, gu_stride, (const bf16*)wd, y, act, N * top, D, F, E, top, limit,
+            alpha, shift, in_wts, st);
     return moe_experts_launch<bf16>((const bf16*)h, ids, (const bf16*)wg, (const bf16*)wu, gu_stride, (const bf16*)wd, y, act,
                                     N, D, F, E, top, limit, alpha, shift, in_wts, st);
 }
