@@ -71,14 +71,14 @@ delta_gates_quads_kernel(const T* __restrict__ qkv, const T* __restrict__ low, i
     for (int p = 0; p < DR_QUADS; p++) {                        // everything is sent for before anything is used
         const int i = (p * 32 + lane) * 4;
         if (i < dim) {
-            dr_load4(w + i, z[p]);
-            dr_load4(dt_bias + (size_t)h * dim + i, dt[p]);
+            mb_load4(w + i, z[p]);
+            mb_load4(dt_bias + (size_t)h * dim + i, dt[p]);
             if (first) {
-                dr_load4(row + (size_t)j * dim + i, a[0][p]);
-                dr_load4(row + ((size_t)G + j) * dim + i, a[1][p]);
+                mb_load4(row + (size_t)j * dim + i, a[0][p]);
+                mb_load4(row + ((size_t)G + j) * dim + i, a[1][p]);
             }
         }
-        if (i < vdim) dr_load4(vs + i, y[p]);
+        if (i < vdim) mb_load4(vs + i, y[p]);
     }
     if (first) {
 #pragma unroll
@@ -101,7 +101,7 @@ delta_gates_quads_kernel(const T* __restrict__ qkv, const T* __restrict__ low, i
                 if (i < dim) {
 #pragma unroll
                     for (int e = 0; e < 4; e++) a[which][p][e] *= r;
-                    dr_store4(dst + i, a[which][p]);
+                    mb_store4(dst + i, a[which][p]);
                 }
             }
         }
@@ -113,12 +113,12 @@ delta_gates_quads_kernel(const T* __restrict__ qkv, const T* __restrict__ low, i
         if (i < vdim) {
 #pragma unroll
             for (int e = 0; e < 4; e++) y[p][e] = dr_silu(y[p][e]);
-            dr_store4(v + (size_t)head * vdim + i, y[p]);
+            mb_store4(v + (size_t)head * vdim + i, y[p]);
         }
         if (i < dim) {
 #pragma unroll
             for (int e = 0; e < 4; e++) z[p][e] = expf(-ea * dr_softplus(z[p][e] + dt[p][e]));
-            dr_store4(g + (size_t)head * dim + i, z[p]);
+            mb_store4(g + (size_t)head * dim + i, z[p]);
         }
     }
     if (lane == 0) beta[head] = dr_sigmoid(mb_load(low + (size_t)n * low_stride + h));
@@ -160,9 +160,9 @@ __global__ void __launch_bounds__(1024) gated_rms_wide_kernel(const float* __res
 #pragma unroll
         for (int e = 0; e < 4; e++) { x[i][e] = z[i][e] = 0.0f; wt[i][e] = 1.0f; }
         if (c < vdim) {
-            dr_load4(o + base + c, x[i]);
-            dr_load4(gp + c, z[i]);
-            if (w) dr_load4(w + (size_t)h * w_head + c, wt[i]);
+            mb_load4(o + base + c, x[i]);
+            mb_load4(gp + c, z[i]);
+            if (w) mb_load4(w + (size_t)h * w_head + c, wt[i]);
         }
 #pragma unroll
         for (int e = 0; e < 4; e++) ss = fmaf(x[i][e], x[i][e], ss);
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(1024) gated_rms_wide_kernel(const float* __res
         const int c = (i * blockDim.x + threadIdx.x) * 4;
 #pragma unroll
         for (int e = 0; e < 4; e++) x[i][e] = x[i][e] * r * wt[i][e] * (silu ? dr_silu(z[i][e]) : dr_sigmoid(z[i][e]));
-        if (c < vdim) dr_store4(out + base + c, x[i]);
+        if (c < vdim) mb_store4(out + base + c, x[i]);
     }
 }
 
@@ -193,9 +193,9 @@ gated_rms_quads_kernel(const float* __restrict__ o, const T* __restrict__ gate, 
 #pragma unroll
         for (int e = 0; e < 4; e++) { x[p][e] = z[p][e] = 0.0f; wt[p][e] = 1.0f; }
         if (c < vdim) {
-            dr_load4(o + (size_t)head * vdim + c, x[p]);
-            dr_load4(gp + c, z[p]);
-            if (w) dr_load4(w + (size_t)h * w_head + c, wt[p]);
+            mb_load4(o + (size_t)head * vdim + c, x[p]);
+            mb_load4(gp + c, z[p]);
+            if (w) mb_load4(w + (size_t)h * w_head + c, wt[p]);
         }
     }
 #pragma unroll
@@ -209,7 +209,7 @@ gated_rms_quads_kernel(const float* __restrict__ o, const T* __restrict__ gate, 
         if (c < vdim) {
 #pragma unroll
             for (int e = 0; e < 4; e++) x[p][e] = x[p][e] * r * wt[p][e] * (silu ? dr_silu(z[p][e]) : dr_sigmoid(z[p][e]));
-            dr_store4(out + (size_t)head * vdim + c, x[p]);
+            mb_store4(out + (size_t)head * vdim + c, x[p]);
         }
     }
 }

@@ -46,23 +46,23 @@ gla_gates_quads_kernel(const T* __restrict__ rows, int stride, const float* __re
     const size_t kd = (size_t)head * dim, vd = (size_t)head * vdim;
     for (int i = lane * 4; i < dim; i += 128) {
         float a[4], b[4], c[4], d[4];
-        dr_load4(row + (size_t)h * dim + i, a);
-        dr_load4(row + (size_t)(H + h) * dim + i, b);
-        dr_load4(z + kd + i, c);
-        dr_load4(zb + (size_t)h * dim + i, d);
+        mb_load4(row + (size_t)h * dim + i, a);
+        mb_load4(row + (size_t)(H + h) * dim + i, b);
+        mb_load4(z + kd + i, c);
+        mb_load4(zb + (size_t)h * dim + i, d);
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             a[e] *= qs;
             c[e] = expf(gs_log_sigmoid(c[e] + d[e]) * inv_tau);
         }
-        dr_store4(q + kd + i, a);
-        dr_store4(k + kd + i, b);
-        dr_store4(g + kd + i, c);
+        mb_store4(q + kd + i, a);
+        mb_store4(k + kd + i, b);
+        mb_store4(g + kd + i, c);
     }
     for (int c = lane * 4; c < vdim; c += 128) {
         float a[4];
-        dr_load4(row + 2 * (size_t)H * dim + (size_t)h * vdim + c, a);
-        dr_store4(v + vd + c, a);
+        mb_load4(row + 2 * (size_t)H * dim + (size_t)h * vdim + c, a);
+        mb_store4(v + vd + c, a);
     }
 }
 
@@ -112,11 +112,11 @@ ssd_gates_quads_kernel(const T* __restrict__ xbc, const float* __restrict__ cb, 
     }
     for (int i = lane * 4; i < len; i += 128) {
         float x[4], c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        dr_load4(row + off + i, x);
-        if (cb) dr_load4(cb + off + i, c);
+        mb_load4(row + off + i, x);
+        if (cb) mb_load4(cb + off + i, c);
 #pragma unroll
         for (int e = 0; e < 4; e++) x[e] = step * dr_silu(x[e] + c[e]);
-        dr_store4(dst + i, x);
+        mb_store4(dst + i, x);
     }
 }
 
@@ -159,9 +159,9 @@ ssd_out_quads_kernel(const float* __restrict__ o, const T* __restrict__ xbc, int
     for (int p = 0; p < SO_QUADS; p++) {
         const int i = (p * 32 + lane) * 4;
         if (i < W) {
-            dr_load4(xbc + (size_t)n * xbc_stride + c0 + i, x[p]);
-            dr_load4(o + (size_t)n * inner + c0 + i, y[p]);
-            dr_load4(z + (size_t)n * z_stride + c0 + i, g[p]);
+            mb_load4(xbc + (size_t)n * xbc_stride + c0 + i, x[p]);
+            mb_load4(o + (size_t)n * inner + c0 + i, y[p]);
+            mb_load4(z + (size_t)n * z_stride + c0 + i, g[p]);
         }
     }
 #pragma unroll
@@ -169,7 +169,7 @@ ssd_out_quads_kernel(const float* __restrict__ o, const T* __restrict__ xbc, int
         const int i = (p * 32 + lane) * 4;
         if (i < W) {
             float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (cb) dr_load4(cb + c0 + i, c);
+            if (cb) mb_load4(cb + c0 + i, c);
             const float d = D[(c0 + i) / P];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
@@ -184,10 +184,10 @@ ssd_out_quads_kernel(const float* __restrict__ o, const T* __restrict__ xbc, int
         const int i = (p * 32 + lane) * 4;
         if (i < W) {
             float c[4];
-            dr_load4(w + c0 + i, c);
+            mb_load4(w + c0 + i, c);
 #pragma unroll
             for (int e = 0; e < 4; e++) y[p][e] = y[p][e] * r * c[e];
-            dr_store4(out + (size_t)n * inner + c0 + i, y[p]);
+            mb_store4(out + (size_t)n * inner + c0 + i, y[p]);
         }
     }
 }

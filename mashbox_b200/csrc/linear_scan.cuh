@@ -9,7 +9,7 @@
 // q and k come per group (G groups, head h reads group h / (H / G)), v per head; everything float32.  See the kernel's
 // own comment for how the work is laid out.
 #pragma once
-#include "common.cuh"
+#include "quads.cuh"
 
 #define DR_THREADS 128
 #define DR_CPT 1            // columns a thread (more: what it reads of q, k, g from shared memory serves them all, but a
@@ -43,23 +43,6 @@ __device__ __forceinline__ void dr_cp4(float* smem, const float* gmem, int size)
 __device__ __forceinline__ float dr_silu(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float dr_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float dr_softplus(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
-
-// four neighbouring values of a row, as floats
-__device__ __forceinline__ void dr_load4(const float* p, float (&x)[4]) {
-    const float4 w = *reinterpret_cast<const float4*>(p);
-    x[0] = w.x; x[1] = w.y; x[2] = w.z; x[3] = w.w;
-}
-__device__ __forceinline__ void dr_load4(const bf16* p, float (&x)[4]) {
-    const uint2 w = *reinterpret_cast<const uint2*>(p);
-    x[0] = __uint_as_float(w.x << 16); x[1] = __uint_as_float(w.x & 0xffff0000u);
-    x[2] = __uint_as_float(w.y << 16); x[3] = __uint_as_float(w.y & 0xffff0000u);
-}
-__device__ __forceinline__ void dr_store4(float* p, const float (&x)[4]) {
-    *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
-}
-__device__ __forceinline__ void dr_store4(bf16* p, const float (&x)[4]) {
-    *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
-}
 
 // The kernels that feed the recurrences and read them come in two forms.  A block per token and head, a value a thread, takes
 // any size; for rows of whole quads (sizes multiples of 4, every row on a 16-byte boundary) a WARP takes a token's head, four

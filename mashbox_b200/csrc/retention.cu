@@ -19,7 +19,7 @@
 //                    from the sequence's own), which gives the part of every o that the segment's own tokens make and
 //                    the state E_j the segment adds; a small kernel chains S0_(j+1) = decay^n S0_j + E_j; a second pass
 //                    adds decay^(t+1) S0_j^T q_t to the t-th token of segment j.  All of it in float32.
-#include "common.cuh"
+#include "quads.cuh"
 
 #define RT_THREADS 128
 #define RT_LANES 8
@@ -61,18 +61,6 @@ __global__ void retention_prep_kernel(const T* __restrict__ rows, int stride, in
 // those pairs of every head it meets (blockDim is a multiple of R / 8, so they are the same pairs); the rest of the row goes
 // through in quads.  R a multiple of 8, sizes multiples of 4, rows on 16-byte boundaries.  2,000 tokens of 16 heads of 128: a
 // sincosf per pair and head 22 us, here 13.
-__device__ __forceinline__ void rt_load4(const float* p, float (&x)[4]) {
-    const float4 w = *reinterpret_cast<const float4*>(p);
-    x[0] = w.x; x[1] = w.y; x[2] = w.z; x[3] = w.w;
-}
-__device__ __forceinline__ void rt_load4(const bf16* p, float (&x)[4]) {
-    const uint2 w = *reinterpret_cast<const uint2*>(p);
-    x[0] = __uint_as_float(w.x << 16); x[1] = __uint_as_float(w.x & 0xffff0000u);
-    x[2] = __uint_as_float(w.y << 16); x[3] = __uint_as_float(w.y & 0xffff0000u);
-}
-__device__ __forceinline__ void rt_store4(float* p, const float (&x)[4]) {
-    *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
-}
 template <typename T>
 __global__ void retention_prep_quads_kernel(const T* __restrict__ rows, int stride, int q_off, int k_off, int v_off,
                                             const int* __restrict__ positions, const float* __restrict__ freqs,
@@ -94,8 +82,8 @@ __global__ void retention_prep_quads_kernel(const T* __restrict__ rows, int stri
             for (int which = 0; which < 2; which++) {
                 float a[4], b[4], x[4], y[4];
                 const T* src = row + (which ? k_off : q_off) + at;
-                rt_load4(src, a);
-                rt_load4(src + half, b);
+                mb_load4(src, a);
+                mb_load4(src + half, b);
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     x[e] = a[e] * c[e] - b[e] * s[e];
@@ -103,8 +91,8 @@ __global__ void retention_prep_quads_kernel(const T* __restrict__ rows, int stri
                     if (which) { x[e] *= k_scale; y[e] *= k_scale; }
                 }
                 float* dst = (which ? kd : qd) + at;
-                rt_store4(dst, x);
-                rt_store4(dst + half, y);
+                mb_store4(dst, x);
+                mb_store4(dst + half, y);
             }
         }
     }
@@ -112,17 +100,17 @@ __global__ void retention_prep_quads_kernel(const T* __restrict__ rows, int stri
     for (int idx = threadIdx.x; idx < H * rest; idx += blockDim.x) {
         const size_t at = (size_t)(idx / rest) * dim + R + (idx % rest) * 4;
         float a[4], b[4];
-        rt_load4(row + q_off + at, a);
-        rt_load4(row + k_off + at, b);
+        mb_load4(row + q_off + at, a);
+        mb_load4(row + k_off + at, b);
 #pragma unroll
         for (int e = 0; e < 4; e++) b[e] *= k_scale;
-        rt_store4(qd + at, a);
-        rt_store4(kd + at, b);
+        mb_store4(qd + at, a);
+        mb_store4(kd + at, b);
     }
     for (int idx = threadIdx.x; idx < H * vdim / 4; idx += blockDim.x) {
         float a[4];
-        rt_load4(row + v_off + idx * 4, a);
-        rt_store4(v + (size_t)n * H * vdim + idx * 4, a);
+        mb_load4(row + v_off + idx * 4, a);
+        mb_store4(v + (size_t)n * H * vdim + idx * 4, a);
     }
 }
 

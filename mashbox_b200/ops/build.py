@@ -60,8 +60,8 @@ LIBRARIES = {            # library name -> (source file, extra compiler flags)
     "sampling_noalloc": ("sampling_noalloc.cu", []),
     "trace": ("trace.cu", []),
 }
-EXTRA_SOURCES = {"sampling_noalloc": ["sampling.cu", "sampling_noalloc.h"], "delta_rule": ["linear_scan.cuh"],
-                 "gated_scan": ["linear_scan.cuh"]}      # files a library includes
+EXTRA_SOURCES = {"sampling_noalloc": ["sampling.cu", "sampling_noalloc.h"], "delta_rule": ["linear_scan.cuh", "quads.cuh"],
+                 "gated_scan": ["linear_scan.cuh", "quads.cuh"], "retention": ["quads.cuh"]}      # files a library includes
 _loaded = {}
 _lock = threading.Lock()
 
