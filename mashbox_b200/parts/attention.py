@@ -202,10 +202,13 @@ class PagedAttention:
         # Sequences of very different lengths, cut into equally many splits, leave the launch waiting for the blocks of the
         # longest one; they are cut in proportion instead where that pays.  Measured on decode steps of 2 to 64 requests of
         # 64 to 16,384 tokens (1B, 3B and 8B shapes, us a layer against the even plan):
-        #   * work for 16 tiles a slot of the device and more: in three rounds of blocks, faster wherever the longest block
-        #     gets shorter (40 requests of 64 to 4,096 tokens: -14; 64: -13; 24 of 64 to 16,384: -144);
-        #   * less: in one round, by how much shorter the longest block gets: by 6 tiles and more +0.1 to -200, by 5 from +0.3
-        #     to -2.9, by 4 and less +0.6 to +6 (splits that meet through global memory cost more than those of a cluster).
+        #   * work for less than 16 tiles a slot of the device: in one round, by how much shorter the longest block gets: by 6
+        #     tiles and more +0.1 to -200, by 5 from +0.3 to -2.9, by 4 and less +0.6 to +6 (splits that meet through global
+        #     memory cost more than those of a cluster);
+        #   * more: in three rounds of blocks, also where the longest block gets up to 1.4 times longer, as long as the even
+        #     plan waits for blocks -- it has more than two rounds of them, or its longest one (with some 11 tiles' time to
+        #     start and finish) runs 1.8 times as long as all slots together -- and not for the memory: 40 requests of 64 to
+        #     4,096 tokens -14, 64 of them -13, 24 of 64 to 16,384 -144; 26 of 4,096 beside 26 of 64, where it does not, +10.
         # The work list is filled up to a coarse grid of lengths with empty items, so that growing sequences seldom change a
         # step's shape; for the same reason every token has a place in the partial buffers, split or not.
         uneven = {}
@@ -219,8 +222,11 @@ class PagedAttention:
                 crowded = sum(lengths) * KV >= 16 * slots
                 cut = uneven_splits(lengths, max(2 * len(decoding), -(-(3 if crowded else 1) * slots // KV)), max_splits)
                 longest = lambda splits: max(-(-t // n) for t, n in zip(lengths, splits))
-                shorter = longest([even_splits(s) for s in decoding]) - longest(cut)
-                if ((choice == "always" or shorter >= (1 if crowded else 6))
+                splits = [even_splits(s) for s in decoding]
+                even, cut_in = longest(splits), longest(cut)
+                waits = sum(splits) * KV > 2 * slots or 5 * (even + 11) * slots >= 9 * sum(lengths) * KV
+                pays = 5 * cut_in <= 7 * even and waits if crowded else cut_in + 6 <= even
+                if ((pays or choice == "always")
                         and ctx.ops.attention_tma_merges(max(listed_items(sum(cut)), max_splits * S + sum(tiles)), KV)):
                     uneven, cluster = dict(zip(decoding, cut)), 0
         for s in range(S):

@@ -37,6 +37,15 @@ def test_batches_that_would_wait_for_one_block_are_cut_in_proportion(lengths):
     assert longest(dec, lengths) < longest(even, lengths)
 
 
+def test_the_cut_stays_while_the_sequences_grow():
+    """37 requests of 190 to 4,400 tokens, whose equal splits would change from two to three on the way"""
+    r = random.Random(3)
+    start = [int(round(np.exp(r.uniform(np.log(128), np.log(4096))))) for _ in range(37)]
+    for t in range(0, 300, 10):
+        p, dec, *_ = T.plan([n + t for n in start] + [1] * 3, [1] * 40, heads=24)
+        assert p["uneven"] and len(dec) == 96
+
+
 def test_random_batches():
     """log-spread lengths: never a longer block than in the plan of equal splits where the device is not crowded, as many places
     in the partial buffers as decode-form tokens, and a work list that grows with the sequences changes its length seldom"""
