@@ -1609,8 +1609,8 @@ def gated_scan(q, k, v, g, o, state, seq, H, G, dim, vdim, per_head, bonus=None,
              dim, vdim, 1 if per_head else 0, 1 if q.shape[0] > 4 * S and not below else 0, int(below), _stream()), "gated_scan")
 
 
-# ---- the linear-attention recurrences over long stretches, 32 tokens at a time (linear_chunks.cu): the sequences of a step
-# that have at least `shortest` tokens, where the step has one (linear_chunks_shortest).
+# ---- the linear-attention recurrences over long stretches, 32 tokens at a time (linear_chunks.cu).  By kind: how long a step's
+# longest sequence has to be for it, where the sequences that long have a block on every SM at most, and where they have more.
 CHUNKS = {"tokens": 80, "delta": (80, 160), "channels": (64, 64), "heads": (80, 80), "wkv": (64, 64), "fixed": (64, 96)}
 CHUNK_MODES = {"delta": 0, "channels": 1, "heads": 2, "wkv": 3, "fixed": 4}
 
@@ -1638,19 +1638,25 @@ def linear_chunks_shortest(lengths, H, dim, vdim, mode):
       100 beside ten of 20 tokens     delta 75/61  heads 77/84  fixed 58/45
       128 beside 37 decoded tokens    delta 75/74  channels 91/133  fixed, 32 heads, 75/61;  200 beside 16: delta 60/94  fixed 50/66
       500 beside sixteen of 60        delta, 24 heads, 323/291  channels 243/338
-    (the scan of the short sequences alone runs the layout for short stretches, which is what channels, heads and wkv gain by)"""
+    (the scan of the short sequences alone runs the layout for short stretches, which is what channels, heads and wkv gain by).
+    Where a step has such a sequence, the others of 32 tokens and more go with it, beside which they cost little: 1,531 + 300 +
+    37 tokens, the 37 by chunks / by the scan: delta 202/220  channels 179/194  heads 196/212  wkv 167/183  fixed 165/179; 500
+    and sixteen of 60: 193/218  159/246  177/224  116/206  113/158.  With the delta rule, whose records are the largest, many
+    of 32 to 47 tokens do not: 500 and sixteen of 33: 191/158, 1,000 and twenty of 50: 269/271."""
     if not linear_chunks_supports(sum(lengths), len(lengths), dim, vdim, mode):
         return 0
     one, more = CHUNKS[mode]
-    shortest = one if sum(n >= one for n in lengths) * H * -(-vdim // 16) <= 148 else more
-    longest, rest = max(lengths), [n for n in lengths if n < shortest]
-    if longest < shortest:
+    least = one if sum(n >= one for n in lengths) * H * -(-vdim // 16) <= 148 else more
+    longest, rest = max(lengths), [n for n in lengths if n < least]
+    if longest < least:
         return 0
     if rest and mode in ("delta", "fixed"):
         pays = longest >= 100 + 3 * len(rest) and 2 * sum(rest) <= 3 * (sum(lengths) - sum(rest))
     else:
         pays = not rest or longest >= 128
-    return shortest if pays else 0
+    if not pays:
+        return 0
+    return 48 if mode == "delta" and sum(32 <= n < 48 for n in lengths) > 2 else 32
 
 
 def linear_chunks_slots(N, S, shortest=32):

@@ -287,7 +287,7 @@ def plan_chunks(ctx, mode, H, dim, vdim):
     shortest = 0 if ctx.dtype != torch.bfloat16 else ctx.ops.linear_chunks_shortest(ctx.q_len, H, dim, vdim, mode)
     rest = shortest > 0 and min(ctx.q_len) < shortest
     ctx.memo[key] = (shortest, rest)
-    code = 1 + 2 * ctx.ops.CHUNKS[mode].index(shortest) + rest if shortest else 0
+    code = 1 + 2 * (shortest > 32) + rest if shortest else 0
     ctx.inputs.add("_".join(map(str, key)), [0] * code)
 
 
@@ -301,7 +301,7 @@ def chunked_recurrence(ctx, mode, q, k, v, g, o, state, H, G, dim, vdim, beta=No
     if not shortest:
         return False
     most = max(ctx.N, ctx.ws.max_rows)
-    floats = ops.linear_chunks_slots(most, max(ctx.S, 64), min(ops.CHUNKS[mode])) * ops.linear_chunks_floats(H, dim, vdim, mode)
+    floats = ops.linear_chunks_slots(most, max(ctx.S, 64)) * ops.linear_chunks_floats(H, dim, vdim, mode)
     scratch = ctx.ws.get("linear_chunks", floats, (), torch.float32, reserve=floats)
     ops.linear_chunks(mode, q, k, v, g, o, state, (ctx.dev("q_start"), ctx.dev("q_len"), ctx.dev("state_slot")), H, G, dim, vdim,
                       beta=beta, scratch=scratch, shortest=shortest, rest=rest)
