@@ -147,11 +147,12 @@ class PagedAttention:
         wide = tc5 and G > DECODE_ROWS
         short = lambda s: wide and not decode_form[s] and ctx.q_len[s] <= DECODE_ROWS
 
-        def key_tiles(s):
+        def keys_of(s):
             hi = ctx.pos0[s] + ctx.q_len[s]
             lo = max(0, ctx.pos0[s] - self.window + 1) if self.window else 0
             front = min(-(-self.keep // KEY_TILE), lo // KEY_TILE)          # tiles of kept positions before the window's
             return front + -(-(hi - lo // KEY_TILE * KEY_TILE) // KEY_TILE)
+        key_tiles = [keys_of(s) for s in range(S)]
 
         # Decode-form sequences on the TMA kernel: when they can all be cut into the same number of splits (set by the
         # longest of them; a shorter one leaves some of its splits empty) the blocks of a sequence and kv head are
@@ -159,12 +160,12 @@ class PagedAttention:
         cluster = 0
         page = ctx.cache.page_size
         if (any(decode_form) and base[True] < target and self._tma(ctx) and ctx.options.get("attention_clusters", True)):
-            raw = min(max_splits, -(-target // base[True]), max(key_tiles(s) for s in range(S) if decode_form[s]) // 2)
+            raw = min(max_splits, -(-target // base[True]), max(key_tiles[s] for s in range(S) if decode_form[s]) // 2)
             want = 1 << (max(1, raw).bit_length() - 1)
             # only when the cluster holds all the splits the launch wants anyway: at one or two sequences (32 and 16
             # splits) more, smaller blocks that meet through global memory are faster than clusters of 8
             most = ctx.ops.attention_tma_max_cluster(self.HD)
-            longest = max(key_tiles(s) for s in range(S) if decode_form[s])
+            longest = max(key_tiles[s] for s in range(S) if decode_form[s])
             if want > most and longest <= 6 * most:
                 # ... unless the sequences are short: up to six key tiles per block, the cheaper meeting of a cluster
                 # outweighs the longer blocks (one sequence of 2,048 keys: 9.2 us in a cluster of 8, 10.4 as 16 splits)
@@ -186,18 +187,20 @@ class PagedAttention:
         if (not cluster and any(decode_form) and self._tma(ctx) and ctx.options.get("attention_splits") is None):
             slots = 2 * ctx.ops.attention_tma_active_clusters(self.HD, 2)
             if slots and 2 * base[True] > slots:
-                work = sum(key_tiles(s) for s in range(S) if decode_form[s]) * KV
+                work = sum(key_tiles[s] for s in range(S) if decode_form[s]) * KV
                 crowd = many_splits(base[True], work, slots, self.HD, min(4, max_splits))
         def even_splits(s):
             if cluster and decode_form[s]:
                 return cluster
-            ns, kv_tiles = 1, key_tiles(s)
+            ns, kv_tiles = 1, key_tiles[s]
             if ctx.q_len[s] <= DECODE_ROWS and base[decode_form[s]] < target and (decode_form[s] or not tc5 or short(s)):
                 ns = max(1, min(max_splits, -(-target // base[decode_form[s]]), kv_tiles // 2))
                 ns = 1 << (ns.bit_length() - 1)                    # a power of two: few distinct work-list shapes
             if decode_form[s] and (crowd or ctx.options.get("attention_splits") is not None):
                 ns = max(1, min(crowd or int(ctx.options["attention_splits"]), kv_tiles // 2))
             return ns
+
+        splits = [even_splits(s) for s in range(S)]
 
         # Sequences of very different lengths, cut into equally many splits, leave the launch waiting for the blocks of the
         # longest one; they are cut in proportion instead where that pays.  Measured on decode steps of 2 to 64 requests of
@@ -216,15 +219,15 @@ class PagedAttention:
         choice = ctx.options.get("attention_uneven_splits", True)         # "always": without the look at what it brings
         if (len(decoding) > 1 and choice and self._tma(ctx) and ctx.options.get("attention_splits") is None
                 and ctx.options.get("attention_cluster_size") is None and ctx.options.get("attention_fused_merge", True)):
-            lengths = [key_tiles(s) for s in decoding]
+            lengths = [key_tiles[s] for s in decoding]
             slots = 2 * ctx.ops.attention_tma_active_clusters(self.HD, 2)
             if slots and 2 * max(lengths) * len(decoding) >= 3 * sum(lengths):
                 crowded = sum(lengths) * KV >= 16 * slots
                 cut = uneven_splits(lengths, max(2 * len(decoding), -(-(3 if crowded else 1) * slots // KV)), max_splits)
-                longest = lambda splits: max(-(-t // n) for t, n in zip(lengths, splits))
-                splits = [even_splits(s) for s in decoding]
-                even, cut_in = longest(splits), longest(cut)
-                waits = sum(splits) * KV > 2 * slots or 5 * (even + 11) * slots >= 9 * sum(lengths) * KV
+                longest = lambda cuts: max(-(-t // n) for t, n in zip(lengths, cuts))
+                equal = [splits[s] for s in decoding]
+                even, cut_in = longest(equal), longest(cut)
+                waits = sum(equal) * KV > 2 * slots or 5 * (even + 11) * slots >= 9 * sum(lengths) * KV
                 pays = 5 * cut_in <= 7 * even and waits if crowded else cut_in + 6 <= even
                 if ((pays or choice == "always")
                         and ctx.ops.attention_tma_merges(max(listed_items(sum(cut)), max_splits * S + sum(tiles)), KV)):
@@ -237,7 +240,7 @@ class PagedAttention:
                     part_tok += [ctx.q_start[s] + t, uneven[s]]
                 dec += [(0, s, 0, sp, uneven[s]) for sp in range(uneven[s])]
                 continue
-            ns = even_splits(s)
+            ns = splits[s]
             if cluster and decode_form[s]:
                 for sp in range(cluster):
                     dec.append((0, s, 0, sp, cluster))
