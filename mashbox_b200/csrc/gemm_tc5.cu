@@ -29,21 +29,14 @@
 #define G_STAGE_BYTES (G_A_BYTES + G_B_BYTES)
 
 // MODE 0: bf16 out (N, M); 1: SwiGLU, W has 2 * M rows, bf16 out (N, M); 2: float out (N, M); 3: bf16 out (N, M) =
-// xIELU of the product (ap z^2 + z / 2 for z > 0, an (e^z - 1 - z) + z / 2 otherwise); 4: as 1 with the gate of routed
-// experts, g = min(gate, ap), u = clamp(up, -ap, ap), out = g sigmoid(an g) (u + shift), gate and up first times the row's
-// row_scale when that is given; 5: bf16 out (N, M) = the square of the product's positive part; 6: as 1 with the tanh form
-// of gelu on the gate.
-//
-// Grouped form (tile_expert given): W is a stack of matrices of `expert_rows` rows each, and every tile of 128 rows of
-// act belongs to one of them -- tile_expert[token tile] says which, -1: the tile holds no rows and is passed over by
-// all three roles alike.  Rows of act are laid out so by whoever sorted them (an expert's rows start at a multiple of
-// 128).  A tile of features that reaches beyond M reads rows of the next matrix of the stack; those columns are not stored.
+// xIELU of the product (ap z^2 + z / 2 for z > 0, an (e^z - 1 - z) + z / 2 otherwise); 4: as 1 with the clamped gate
+// g = min(gate, ap), u = clamp(up, -ap, ap), out = g sigmoid(an g) (u + shift); 5: bf16 out (N, M) = the square of the product's
+// positive part; 6: as 1 with the tanh form of gelu on the gate.
 template <int MODE>
 __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant__ CUtensorMap amap,
                                                            const __grid_constant__ CUtensorMap wmap,
                                                            void* __restrict__ out, int N, int M, int K, float ap,
-                                                           float an, float shift, int* err, const int* __restrict__ tile_expert,
-                                                           int expert_rows, const float* __restrict__ row_scale) {
+                                                           float an, float shift, int* err) {
     constexpr bool GATED = MODE == 1 || MODE == 4 || MODE == 6;
     constexpr int FEATS = GATED ? 128 : 256;              // output features of one tile
     extern __shared__ unsigned char smem_unaligned[];
@@ -55,7 +48,6 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * G_STAGES;
     const uint32_t tfull0 = empty0 + 8 * G_STAGES, tempty0 = tfull0 + 16;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    __shared__ int used;
 
     if (tid == 0) {
         for (int s = 0; s < G_STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
@@ -67,22 +59,10 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
         tmem_alloc(smem_u32(tmem_slot), 512);
         tmem_relinquish();
     }
-    // Grouped: the tiles that hold rows come first; only those are dealt out.  (Dealt out with the empty ones among them, the
-    // blocks got 6 to 12 tiles of work each: 2,000 tokens of 6 of 64 experts, K 2,048, 2 x 1,408 features: 237 us, now
-    // 227; the down product 140, now 138.)
-    int tok_tiles = (N + G_BM - 1) / G_BM;
-    if (tile_expert) {
-        if (tid == 0) used = 0;
-        __syncthreads();
-        int last = 0;
-        for (int t = tid; t < tok_tiles; t += blockDim.x) if (tile_expert[t] >= 0) last = t + 1;
-        if (last) atomicMax(&used, last);
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (tile_expert) tok_tiles = used;
-    const int m_tiles = (M + FEATS - 1) / FEATS, tiles = tok_tiles * m_tiles, kblocks = (K + G_BK - 1) / G_BK;
+    const int tok_tiles = (N + G_BM - 1) / G_BM, m_tiles = (M + FEATS - 1) / FEATS, tiles = tok_tiles * m_tiles, kblocks = (K + G_BK - 1) / G_BK;
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -90,12 +70,6 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
             int it = 0;                                               // stages issued so far
             for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
                 const int tok0 = (tile % tok_tiles) * G_BM, m0 = (tile / tok_tiles) * FEATS;
-                int wrow = 0;
-                if (tile_expert) {
-                    const int e = tile_expert[tile % tok_tiles];
-                    if (e < 0) continue;
-                    wrow = e * expert_rows;
-                }
                 bool ok = true;
                 for (int kb = 0; kb < kblocks && ok; kb++, it++) {
                     const int s = it % G_STAGES, round = it / G_STAGES;
@@ -103,8 +77,8 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
                     const uint32_t fb = full0 + 8 * s, a_dst = stage0 + s * G_STAGE_BYTES, b_dst = a_dst + G_A_BYTES;
                     mbar_expect_tx(fb, G_STAGE_BYTES);
                     tma_load_2d(a_dst, &amap, kb * G_BK, tok0, fb);
-                    tma_load_2d(b_dst, &wmap, kb * G_BK, wrow + m0, fb);
-                    tma_load_2d(b_dst + G_B_BYTES / 2, &wmap, kb * G_BK, wrow + (GATED ? M + m0 : m0 + 128), fb);
+                    tma_load_2d(b_dst, &wmap, kb * G_BK, m0, fb);
+                    tma_load_2d(b_dst + G_B_BYTES / 2, &wmap, kb * G_BK, GATED ? M + m0 : m0 + 128, fb);
                 }
                 if (!ok) break;
             }
@@ -114,7 +88,6 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
             constexpr uint32_t idesc = umma_idesc(G_BM, G_BN);
             int it = 0, j = 0;                                        // stages consumed, tiles done by this block
             for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-                if (tile_expert && tile_expert[tile % tok_tiles] < 0) continue;
                 const int acc = j & 1, use = j >> 1;
                 j++;
                 if (use > 0 && !mbar_wait(tempty0 + 8 * acc, (use - 1) & 1, err)) break;
@@ -140,14 +113,12 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
         const int q = warp & 3;                                       // the 32 TMEM lanes this warp may read
         int j = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            if (tile_expert && tile_expert[tile % tok_tiles] < 0) continue;
             const int acc = j & 1, use = j >> 1;
             j++;
             if (!mbar_wait(tfull0 + 8 * acc, use & 1, err)) break;
             tc_fence_after();
             const int tok = (tile % tok_tiles) * G_BM + q * 32 + lane, m0 = (tile / tok_tiles) * FEATS;
             const uint32_t taddr = tmem_base + acc * G_BN + ((uint32_t)(q * 32) << 16);
-            const float rs = MODE == 4 && row_scale && tok < N ? row_scale[tok] : 1.0f;
 #pragma unroll 1
             for (int c = 0; c < FEATS; c += 32) {
                 uint32_t r[32];
@@ -159,8 +130,8 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
 #pragma unroll
                     for (int i = 0; i < 32; i++) {
                         // gate and up pass through bf16 as they do when the products are separate kernels
-                        float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[i]) * rs));
-                        float up = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[i]) * rs));
+                        float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r[i])));
+                        float up = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[i])));
                         if (MODE == 4) {
                             g = fminf(g, ap);
                             up = fminf(fmaxf(up, -ap), ap) + shift;
@@ -232,8 +203,7 @@ __global__ void __launch_bounds__(192, 1) gemm_tc5_kernel(const __grid_constant_
 
 template <int MODE>
 static int tc5_launch(const void* act, const void* W, void* out, int N, int M, int K, int* err, cudaStream_t st,
-                      float ap = 0.0f, float an = 0.0f, const int* tile_expert = nullptr, int experts = 1,
-                      float shift = 1.0f, const float* row_scale = nullptr) {
+                      float ap = 0.0f, float an = 0.0f, float shift = 1.0f) {
     if (N == 0 || M == 0) return 0;
     if (K % 8 || M % 8 || K < 8 || (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(act) & 15) ||
         (reinterpret_cast<uintptr_t>(out) & 15))
@@ -242,8 +212,7 @@ static int tc5_launch(const void* act, const void* W, void* out, int N, int M, i
     int rc = matrix_map(act, N, K, 128, &amap);
     if (rc) return rc;
     constexpr int PER = (MODE == 1 || MODE == 4 || MODE == 6) ? 2 : 1;
-    if (tile_expert && (experts < 1 || N % G_BM)) return -2;
-    rc = matrix_map(W, (long long)PER * M * experts, K, 128, &wmap);
+    rc = matrix_map(W, (long long)PER * M, K, 128, &wmap);
     if (rc) return rc;
     const size_t smem = 1024 + (size_t)G_STAGES * G_STAGE_BYTES + (2 * G_STAGES + 4) * 8 + 16;
     static bool configured = false;
@@ -259,8 +228,7 @@ static int tc5_launch(const void* act, const void* W, void* out, int N, int M, i
     }
     const int feats = PER == 2 ? 128 : 256;
     const int tiles = ((N + G_BM - 1) / G_BM) * ((M + feats - 1) / feats);
-    gemm_tc5_kernel<MODE><<<tiles < sms ? tiles : sms, 192, smem, st>>>(amap, wmap, out, N, M, K, ap, an, shift, err, tile_expert,
-                                                                        PER * M, row_scale);
+    gemm_tc5_kernel<MODE><<<tiles < sms ? tiles : sms, 192, smem, st>>>(amap, wmap, out, N, M, K, ap, an, shift, err);
     MB_LAUNCH_CHECK();
     return 0;
 }
@@ -295,25 +263,9 @@ MB_API int mb_gemm_tc5_f32out(const void* act, const void* W, void* out, int N, 
     return tc5_launch<2>(act, W, out, N, M, K, err, st);
 }
 
-
-// Grouped forms: act (N, K) with N a multiple of 128, every 128 rows one expert's (tile_expert[N / 128]: its index, -1:
-// no rows); W a stack of `experts` matrices.  Gated: (experts, 2 M, K), gate rows then up rows of each expert,
-// out (N, M) bf16 = g sigmoid(alpha g) (u + shift) with g = min(gate, limit), u = clamp(up, -limit, limit); row_scale (N
-// floats, or null): every row's gate and up are multiplied by its number first (the row's input times that number).
-MB_API int mb_gemm_tc5_grouped_gated_bf16(const void* act, const void* W, void* out, int N, int M, int K,
-                                          const int* tile_expert, int experts, float limit, float alpha, float shift,
-                                          const float* row_scale, int* err, cudaStream_t st) {
-    if (!tile_expert) return -2;
-    return tc5_launch<4>(act, W, out, N, M, K, err, st, limit, alpha, tile_expert, experts, shift, row_scale);
-}
-// The same gate as a dense layer's: W (2 M, K) = [gate rows | up rows], any N; limit <= 0: no clamps.
+// W (2 M, K) = [gate rows | up rows]; out (N, M) = g sigmoid(alpha g) (u + shift), g = min(gate, limit), u = clamp(up, -limit,
+// limit); limit <= 0: no clamps.
 MB_API int mb_gemm_tc5_glu_clamped_bf16(const void* act, const void* W, void* out, int N, int M, int K, float limit,
                                         float alpha, float shift, int* err, cudaStream_t st) {
-    return tc5_launch<4>(act, W, out, N, M, K, err, st, limit > 0.0f ? limit : 3.0e38f, alpha, nullptr, 1, shift);
-}
-// W (experts, M, K); out (N, M) float32
-MB_API int mb_gemm_tc5_grouped_f32out(const void* act, const void* W, void* out, int N, int M, int K, const int* tile_expert,
-                                      int experts, int* err, cudaStream_t st) {
-    if (!tile_expert) return -2;
-    return tc5_launch<2>(act, W, out, N, M, K, err, st, 0.0f, 0.0f, tile_expert, experts);
+    return tc5_launch<4>(act, W, out, N, M, K, err, st, limit > 0.0f ? limit : 3.0e38f, alpha, shift);
 }

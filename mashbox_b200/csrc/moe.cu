@@ -696,13 +696,14 @@ MB_API int mb_moe_grouped_bf16(const void* h, const int* ids, const void* wg, co
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Steps of 128 tokens and more (bf16) hand the two products to the tcgen05 product in its grouped form, which wants the
-// rows of every expert side by side, starting at a multiple of 128:
-//   moe_sort_padded   one block: per pair its row in that layout (`place`), per tile of 128 rows its expert (-1: empty)
+// Steps of 128 tokens and more (bf16) hand the two products to gemm_experts.cu, which wants the rows of every expert side by
+// side, starting at a multiple of 128:
+//   moe_sort_padded   one block: per pair its row in that layout (`place`), per tile of 128 rows what starts there (`groups`:
+//                     expert | rows << 12 for up to 256 rows of an expert, -1: nothing)
 //   moe_gather_rows   h rows, by token, to their places
 //   moe_combine_rows  out[n] = sum over the places, in order, of weight * y[place of (n, k)]
 __global__ void moe_sort_padded_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ place,
-                                       int* __restrict__ tile_expert, int max_tiles) {
+                                       int* __restrict__ groups, int max_tiles) {
     extern __shared__ int sh[];
     int* cnt = sh;              // E
     int* start = sh + E;        // E + 1, in tiles
@@ -720,10 +721,10 @@ __global__ void moe_sort_padded_kernel(const int* __restrict__ ids, int P, int E
         start[E] = t;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < max_tiles; t += blockDim.x) tile_expert[t] = -1;
+    for (int t = threadIdx.x; t < max_tiles; t += blockDim.x) groups[t] = -1;
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        for (int t = start[e]; t < start[e + 1] && t < max_tiles; t++) tile_expert[t] = e;
+        for (int t = start[e]; t < start[e + 1] && t < max_tiles; t += 2) groups[t] = e | min(256, cnt[e] - (t - start[e]) * 128) << 12;
         cnt[e] = start[e] * 128;                    // from here on: the next free row of the expert
     }
     __syncthreads();
@@ -782,14 +783,14 @@ moe_combine_quads_kernel(const float* __restrict__ y, const int* __restrict__ pl
     }
 }
 
-// place (N top), tile_expert (N top / 128 + E), rows ((N top / 128 + E) 128, D) bf16
-MB_API int mb_moe_sort_gather(const void* h, const int* ids, int* place, int* tile_expert, void* rows, int N, int D, int E,
+// place (N top), groups (N top / 128 + E), rows ((N top / 128 + E) 128, D) bf16
+MB_API int mb_moe_sort_gather(const void* h, const int* ids, int* place, int* groups, void* rows, int N, int D, int E,
                               int top, const float* in_wts, float* row_scale, cudaStream_t st) {
     if (N == 0) return 0;
     const long long P = (long long)N * top;
     if (D % 8 || D < 8 || E < 1 || E > 4096 || P > (1 << 24) || (row_scale && !in_wts)) return -2;
     const int max_tiles = (int)(P / 128) + E;
-    moe_sort_padded_kernel<<<1, 1024, (size_t)(2 * E + 1) * sizeof(int), st>>>(ids, (int)P, E, place, tile_expert, max_tiles);
+    moe_sort_padded_kernel<<<1, 1024, (size_t)(2 * E + 1) * sizeof(int), st>>>(ids, (int)P, E, place, groups, max_tiles);
     MB_LAUNCH_CHECK();
     moe_gather_rows_kernel<<<(unsigned)P, 128, 0, st>>>((const bf16*)h, place, (bf16*)rows, D, top, in_wts, row_scale);
     MB_LAUNCH_CHECK();

@@ -753,7 +753,7 @@ def moe_grouped(h, ids, wg, wu, wd, y, act, scratch, limit, alpha, shift=1.0, in
 
 
 def moe_tc5_supports(N, D, F, dtype):
-    """steps of 128 tokens and more: the experts' products run on the tcgen05 product in its grouped form"""
+    """steps of 128 tokens and more: the experts' products run on tcgen05 tiles (gemm_experts.cu)"""
     return dtype == torch.bfloat16 and N >= 128 and D % 8 == 0 and F % 8 == 0 and TC5["experts"]
 
 
@@ -777,17 +777,17 @@ def moe_tc5(h, ids, wts, wgu, wd, out, rows, act, y, scratch, limit, alpha, shif
     if rows.shape[0] < 128 * T or act.shape[0] < 128 * T or y.shape[0] < 128 * T or scratch.numel() < N * top + T \
             or (row_scale is not None and row_scale.numel() < 128 * T):
         raise KernelError("moe_tc5: the working memory is too small")
-    place, tile_expert = scratch[:N * top], scratch[N * top:N * top + T]
+    place, groups = scratch[:N * top], scratch[N * top:N * top + T]
     f = _fn("moe", "mb_moe_sort_gather", [c_void_p] * 5 + [c_int] * 4 + [c_void_p] * 3)
-    _check(f(_p(h), _p(ids), _p(place), _p(tile_expert), _p(rows), N, D, E, top, _p(wts), _p(row_scale), _stream()),
+    _check(f(_p(h), _p(ids), _p(place), _p(groups), _p(rows), N, D, E, top, _p(wts), _p(row_scale), _stream()),
            "moe_sort_gather")
     err = error_word(h.device)
-    f = _fn("gemm_tc5", "mb_gemm_tc5_grouped_gated_bf16",
+    f = _fn("gemm_experts", "mb_gemm_experts_gated_bf16",
             [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_int, c_float, c_float, c_float, c_void_p, c_void_p, c_void_p])
-    _check(f(_p(rows), _p(wgu), _p(act), 128 * T, F, D, _p(tile_expert), E, float(limit), float(alpha), float(shift),
-             _p(row_scale), _p(err), _stream()), "gemm_tc5_grouped_gated")
-    f = _fn("gemm_tc5", "mb_gemm_tc5_grouped_f32out", [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_int, c_void_p, c_void_p])
-    _check(f(_p(act), _p(wd), _p(y), 128 * T, D, F, _p(tile_expert), E, _p(err), _stream()), "gemm_tc5_grouped")
+    _check(f(_p(rows), _p(wgu), _p(act), 128 * T, F, D, _p(groups), E, float(limit), float(alpha), float(shift),
+             _p(row_scale), _p(err), _stream()), "gemm_experts_gated")
+    f = _fn("gemm_experts", "mb_gemm_experts_f32out", [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_int, c_void_p, c_void_p])
+    _check(f(_p(act), _p(wd), _p(y), 128 * T, D, F, _p(groups), E, _p(err), _stream()), "gemm_experts")
     f = _fn("moe", "mb_moe_combine_rows", [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_void_p, c_int, c_void_p])
     _check(f(_p(y), _p(place), _p(wts if row_scale is None else None), _p(out), N, D, top, _p(shared), _p(gate), gate.stride(0) if gate is not None else 0,
              _stream()), "moe_combine_rows")

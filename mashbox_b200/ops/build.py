@@ -27,6 +27,7 @@ LIBRARIES = {            # library name -> (source file, extra compiler flags)
     "elementwise": ("elementwise.cu", []),
     "gemm_f32": ("gemm_f32.cu", []),
     "gemm_tc5": ("gemm_tc5.cu", []),
+    "gemm_experts": ("gemm_experts.cu", []),                           # routed experts, weights on the M side
     "gemm_stream": ("gemm_stream.cu", []),
     "gemv": ("gemv.cu", []),
     "attention_simple": ("attention_simple.cu", []),
