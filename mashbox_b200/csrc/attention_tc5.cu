@@ -11,7 +11,7 @@
 //              warpgroup also fetches its query tile of the NEXT unit before this unit's output is written.
 //   warp 8     producer: walks the block table and brings each K and V tile in with one cp.async.bulk.tensor.2d per
 //              page and 64-column half (128-byte swizzle), one lane per box, page ids read one tile ahead; two stages.
-//   warp 9     one thread issues the products, for the two query tiles in turn: O_g += P_g V (M = 128 rows, N = head
+//   warp 9     one lane issues the products, for the two query tiles in turn: O_g += P_g V (M = 128 rows, N = head
 //              size, 8 k-steps over the keys; V is the MN-major operand, read as the TMA laid it out), then
 //              S_g = Q_g K^T of the next key tile (M = 128, N = 128 keys, head size / 16 k-steps), so the products of
 //              one query tile run under the softmax of the other.
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) attn_tc5_kernel(const AttnParam
                    s_full0 = k_full0 + 64, p_full0 = k_full0 + 80, o_done0 = k_full0 + 96, q_ready0 = k_full0 + 112,
                    a1_ready = k_full0 + 128, o1_read = k_full0 + 136;       // differential form: map 1 handed over / read
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
     if (tid == 8 * 32) {
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(&kmap) : "memory");
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(&vmap) : "memory");
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(T5_THREADS, 1) attn_tc5_kernel(const AttnParam
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = warp_uniform(*tmem_slot);
     // tensor memory: scores of tile g in columns g*128 .. +127 (its probabilities go back into the first 64 of them as
     // bf16 pairs), output accumulator of tile g in columns 256 + g*HD .. +HD-1
     const uint32_t tm_s0 = tmem_base, tm_o0 = tmem_base + 256;
@@ -282,11 +282,13 @@ __global__ void __launch_bounds__(T5_THREADS, 1) attn_tc5_kernel(const AttnParam
         }
     } else if (warp == 9) {
         // ---------------------------------------------------------------- products
-        // One thread issues, for the two query tiles in turn: O_g += P_g(t) V(t), then S_g = Q_g K(t+1)^T.  While the
+        // One lane issues (umma_f16_warp), for the two query tiles in turn: O_g += P_g(t) V(t), then S_g = Q_g K(t+1)^T.  While the
         // softmax warps of one tile work, the tensor cores run the products of the other.  The score product of a tile
         // overwrites the buffer its probabilities lay in; it is issued after the output product that read them, and the
-        // products run in the order they were issued.
-        if (lane == 0) {
+        // products run in the order they were issued.  (Issued in a branch of one lane the twelve instructions of a tile and
+        // their commits bounded the block, not the softmax: without its exponentials it took as long.  2,048 tokens at 14,336,
+        // us: head size 64 475 -> 422; at 6,144: 235 -> 206, head size 128 264 -> 218.)
+        {
             // D float, A and B bf16, M = 128; scores N = 128 keys, outputs N = HD with B MN-major (bit 16)
             constexpr uint32_t idesc_qk = umma_idesc(T5_BM, T5_BN);
             constexpr uint32_t idesc_pv = umma_idesc(T5_BM, HD) | (1u << 16);
@@ -295,14 +297,16 @@ __global__ void __launch_bounds__(T5_THREADS, 1) attn_tc5_kernel(const AttnParam
             bool live = unit >= 0 && t5_unit(P, unit, U);
             int kt = 0, nu0 = 0, nu1 = 0, nt0 = 0, nt1 = 0;           // key tiles; per query tile: units and tiles so far
             bool ok = true;
+            auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, P.err)); };
             for (; ok && unit >= 0; k++, unit = t5_unit_at(k, n_units), live = unit >= 0 && t5_unit(P, unit, U)) {
                 if (!live) continue;
+                const int T = warp_uniform(U.T), T0 = warp_uniform(U.T0), T1 = warp_uniform(U.T1);
                 auto last_reader = [&](int g, int t) -> bool {      // no later query tile reads key tile t
-                    return g == T5_QT - 1 || t >= U.T1;
+                    return g == T5_QT - 1 || t >= T1;
                 };
                 auto scores = [&](int g, int t) -> bool {           // S_g = Q_g K_t^T
                     const int n = kt + t, s = n & 1;
-                    if (!mbar_wait(k_full0 + 8 * s, (n >> 1) & 1, P.err)) return false;
+                    if (!wait(k_full0 + 8 * s, (n >> 1) & 1)) return false;
                     tc_fence_after();
                     const uint32_t k_lo = umma_desc_lo(k_s0 + s * TILE, 0), q_lo = umma_desc_lo(q_s0 + g * TILE, 0);
 #ifdef T5_DIFF
@@ -314,44 +318,44 @@ __global__ void __launch_bounds__(T5_THREADS, 1) attn_tc5_kernel(const AttnParam
                     for (int ks = ks0; ks < ks1; ks++) {
                         constexpr uint32_t half = T5_HALF >> 4;
                         const uint32_t off = (ks >> 2) * half + (ks & 3) * 2;             // in 16-byte units
-                        umma_f16(tm_s0 + g * 128, umma_desc_join(q_lo + off), umma_desc_join(k_lo + off), idesc_qk, ks > ks0);
+                        umma_f16_warp(tm_s0 + g * 128, umma_desc_join(q_lo + off), umma_desc_join(k_lo + off), idesc_qk, ks > ks0);
                     }
-                    if (last_reader(g, t)) umma_commit(k_empty0 + 8 * s);
-                    umma_commit(s_full0 + 8 * g);
+                    if (last_reader(g, t)) umma_commit_warp(k_empty0 + 8 * s);
+                    umma_commit_warp(s_full0 + 8 * g);
                     return true;
                 };
                 auto outputs = [&](int g, int t) -> bool {          // O_g += P_g V_t
                     const int n = kt + t, s = n & 1;
-                    if (!mbar_wait(p_full0 + 8 * g, ((g == 0 ? nt0 : nt1) + t) & 1, P.err)) return false;
-                    if (!mbar_wait(v_full0 + 8 * s, (n >> 1) & 1, P.err)) return false;
+                    if (!wait(p_full0 + 8 * g, ((g == 0 ? nt0 : nt1) + t) & 1)) return false;
+                    if (!wait(v_full0 + 8 * s, (n >> 1) & 1)) return false;
                     tc_fence_after();
                     const uint32_t v_lo = umma_desc_lo(v_s0 + s * TILE, T5_HALF);
 #pragma unroll
                     for (int kk = 0; kk < 8; kk++)                  // 16 keys per step: 2,048 bytes further in the tile
-                        umma_f16_ts(tm_o0 + g * HD, tm_s0 + g * 128 + kk * 8, umma_desc_join(v_lo + kk * 128), idesc_pv,
+                        umma_f16_ts_warp(tm_o0 + g * HD, tm_s0 + g * 128 + kk * 8, umma_desc_join(v_lo + kk * 128), idesc_pv,
                                     (t > 0 || kk > 0) ? 1u : 0u);
 #ifdef T5_SIG
 #pragma unroll
                     for (int kk = 0; kk < 8; kk++)                  // the low parts of the weights, from the last 64 columns
-                        umma_f16_ts(tm_o0 + g * HD, tm_s0 + g * 128 + 64 + kk * 8, umma_desc_join(v_lo + kk * 128), idesc_pv, 1u);
+                        umma_f16_ts_warp(tm_o0 + g * HD, tm_s0 + g * 128 + 64 + kk * 8, umma_desc_join(v_lo + kk * 128), idesc_pv, 1u);
 #endif
-                    if (last_reader(g, t)) umma_commit(v_empty0 + 8 * s);
-                    if (t == U.tiles(g) - 1) umma_commit(o_done0 + 8 * g);
+                    if (last_reader(g, t)) umma_commit_warp(v_empty0 + 8 * s);
+                    if (t == (g == 0 ? T0 : T1) - 1) umma_commit_warp(o_done0 + 8 * g);
                     return true;
                 };
 #pragma unroll
                 for (int g = 0; g < T5_QT; g++)
-                    if (ok && U.tiles(g) > 0) ok = mbar_wait(q_ready0 + 8 * g, (g == 0 ? nu0 : nu1) & 1, P.err) && scores(g, 0);
-                for (int t = 0; t < U.T && ok; t++) {
+                    if (ok && (g == 0 ? T0 : T1) > 0) ok = wait(q_ready0 + 8 * g, (g == 0 ? nu0 : nu1) & 1) && scores(g, 0);
+                for (int t = 0; t < T && ok; t++) {
 #pragma unroll
                     for (int g = 0; g < T5_QT; g++) {
-                        if (ok && t < U.tiles(g)) ok = outputs(g, t);
-                        if (ok && t + 1 < U.tiles(g)) ok = scores(g, t + 1);
+                        if (ok && t < (g == 0 ? T0 : T1)) ok = outputs(g, t);
+                        if (ok && t + 1 < (g == 0 ? T0 : T1)) ok = scores(g, t + 1);
                     }
                 }
-                kt += U.T;
-                if (U.T0 > 0) { nu0++; nt0 += U.T0; }
-                if (U.T1 > 0) { nu1++; nt1 += U.T1; }
+                kt += T;
+                if (T0 > 0) { nu0++; nt0 += T0; }
+                if (T1 > 0) { nu1++; nt1 += T1; }
             }
         }
     }
