@@ -1,0 +1,415 @@
+// True 32-bit matrix product on the tensor cores: C[n, m] = sum_k A[n, k] * W[m, k], float32 operands and results.
+//
+// Every float32 operand is cut into three bf16 numbers that add up to it exactly, x = h + m + l (h its upper 8 significant
+// bits, m the rest rounded to 8, l what is left), so a product is a sum of exact bf16 products; the six that matter --
+// m m, h l, l h, h m, m h and h h, in this order; m l, l m and l l lie below 2^-24 of the product -- run as tcgen05.mma
+// (kind::f16, float accumulator).  The tensor cores cut off the low bits of what they add to an accumulator instead of
+// rounding it, so an accumulator never grows old: it takes ONE block of 32 k (twelve instructions, the small parts
+// first, the two that carry the result last) and is then added, rounded to nearest, to a sum in registers.  Measured against
+// 64 bits this is nearer than one chain of fused multiply-adds over k (gemm_f32.cu): relative error 0.8e-7 / 1.1e-7 / 1.7e-7 at
+// K 512 / 2,048 / 8,192 on normal values, the chain's 4e-7 / 8e-7 / 16e-7 (tests/test_float32_split_gpu.py).  The FMA units' product
+// at the same size and this one: 509 x 16384 x 2048 684 -> 243 us, 509 x 2048 x 8192 494 -> 102, 1 x 2048 x 8192
+// 405 -> 65; one row of a head of 128,256 alone is slower (333 -> 415).
+//
+// An output is the same operations in the same order however many rows a call has: blocks of 32 k in ascending order
+// within a quarter of K, the quarters' sums in ascending order.  Tiles, and whether one block or a cluster of four goes
+// through the quarters, change no bit.
+//
+// One block: 128 rows of W (the M side of the instructions) x TN rows of A, warp-specialised:
+//   warp 0      TMA: 128 x 32 floats of W per stage into a ring of 4
+//   warp 2      TMA: the three bf16 planes of TN x 32 values of A (64-byte swizzle), cut by split_rows_kernel beforehand:
+//               they are read once per tile of W, W once per tile of A
+//   warps 4-7   cut a stage of W into its three planes in shared memory, as the instructions want them
+//   warp 1      one lane issues the products; accumulators of TN columns, two in turn
+//   warps 8-15  add a block's accumulator to the sums in registers (thread = a row of W, half of the columns)
+// A cluster of four blocks takes a quarter of K each where the tiles alone leave the device idle: the sums meet in
+// shared memory.  A single block puts the sum of a quarter down in C and adds the next to it.
+//
+// A result that is not finite is computed again as one chain of fused multiply-adds, so infinities and NaN come out as the
+// plain product has them (an infinite operand has no such parts).
+#include "tcgen05.cuh"
+
+MB_PDL_SWITCH(mb_gemm_f32_tc5_set_pdl)              // the product starts, and brings W in, while the planes are cut
+
+#define FS_BK 32                                   // k of a stage and of an accumulator
+#define FS_RAW 4                                   // stages of W as it comes
+#define FS_RAW_BYTES (128 * FS_BK * 4)
+#define FS_W_PLANE (128 * FS_BK * 2)
+#define FS_THREADS 512
+
+template <int TN> struct FsShape {
+    static constexpr int X_PLANE = TN * FS_BK * 2;
+    static constexpr int STAGE = 3 * FS_W_PLANE + 3 * X_PLANE;
+    static constexpr int STAGES = TN == 256 ? 2 : TN == 128 ? 3 : 4;
+    static constexpr int TMEM = 2 * TN < 32 ? 32 : 2 * TN;
+    static constexpr int SMEM = 1024 + STAGES * STAGE + FS_RAW * FS_RAW_BYTES + 256;
+};
+
+// four floats -> their three bf16 parts, two to a word.  h is cut off (never rounded up to infinity), m is rounded, l is exact.
+__device__ __forceinline__ void fs_split4(const float4 x, uint2& h, uint2& m, uint2& l) {
+    const uint32_t a = __float_as_uint(x.x), b = __float_as_uint(x.y), c = __float_as_uint(x.z), d = __float_as_uint(x.w);
+    h.x = __byte_perm(a, b, 0x7632);
+    h.y = __byte_perm(c, d, 0x7632);
+    const float ra = x.x - __uint_as_float(a & 0xffff0000u), rb = x.y - __uint_as_float(b & 0xffff0000u);
+    const float rc = x.z - __uint_as_float(c & 0xffff0000u), rd = x.w - __uint_as_float(d & 0xffff0000u);
+    m.x = pack_bf16(ra, rb);
+    m.y = pack_bf16(rc, rd);
+    l.x = pack_bf16(ra - __uint_as_float(m.x << 16), rb - __uint_as_float(m.x & 0xffff0000u));
+    l.y = pack_bf16(rc - __uint_as_float(m.y << 16), rd - __uint_as_float(m.y & 0xffff0000u));
+}
+
+// A (N, K) -> planes (3, N, Kp) bf16, Kp = K rounded up to 8, zeros behind K.  A thread cuts four values.
+template <bool VEC>
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, bf16* __restrict__ planes, int N, int K, int Kp) {
+    const int quads = Kp / 4;
+    const size_t total = (size_t)N * quads, plane = (size_t)N * Kp;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {
+        const int n = (int)(i / quads), k = (int)(i % quads) * 4;
+        const float* p = A + (size_t)n * K + k;
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (k < K) x = VEC ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+        uint2 h, m, l;
+        fs_split4(x, h, m, l);
+        uint2* o = reinterpret_cast<uint2*>(planes + (size_t)n * Kp + k);
+        o[0] = h;
+        o[plane / 4] = m;
+        o[plane / 2] = l;
+    }
+    pdl_launch_dependents();
+}
+
+// the shared-memory descriptor of a K-major tile of 64-byte rows with the 64-byte swizzle (8 rows 512 bytes apart, version 1, layout
+// type 4): only its low word, the address in units of 16 bytes, differs from product to product
+__device__ __forceinline__ uint64_t fs_desc(uint32_t lo) {
+    constexpr uint32_t HI = (512u >> 4) | (1u << 14) | (4u << 29);
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(d) : "r"(lo), "r"(HI));
+    return d;
+}
+
+__device__ __forceinline__ void fs_ld8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+}
+
+__device__ __noinline__ float fs_plain_chain(const float* a, const float* w, int K) {
+    float s = 0.0f;
+    for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
+    return s;
+}
+__device__ __forceinline__ bool fs_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u; }
+
+__device__ __forceinline__ float fs_ld_cluster(uint32_t addr, int rank) {
+    uint32_t at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void fs_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// CL blocks of a cluster: 1 (the block goes through all of K) or 4 (block r through the r-th quarter)
+template <int TN, int CL>
+__global__ void __launch_bounds__(FS_THREADS, 1)
+gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const float* __restrict__ A,
+                    const float* __restrict__ W, float* C, int N, int M, int K, int ldc, int* err) {
+    using S = FsShape<TN>;
+    constexpr int HALF = TN / 2;                               // columns of a warp of the last two groups
+    extern __shared__ unsigned char smem_unaligned[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
+    const uint32_t stage0 = smem_u32(smem), raw0 = stage0 + S::STAGES * S::STAGE;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::STAGES * S::STAGE + FS_RAW * FS_RAW_BYTES);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * S::STAGES, rfull0 = empty0 + 8 * S::STAGES,
+                   rempty0 = rfull0 + 8 * FS_RAW, tfull0 = rempty0 + 8 * FS_RAW, tempty0 = tfull0 + 16;
+    const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
+
+    if (tid == 0) {
+        for (int s = 0; s < S::STAGES; s++) { mbar_init(full0 + 8 * s, 5); mbar_init(empty0 + 8 * s, 1); }
+        for (int s = 0; s < FS_RAW; s++) { mbar_init(rfull0 + 8 * s, 1); mbar_init(rempty0 + 8 * s, 4); }
+        for (int a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 8); }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), S::TMEM);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = warp_uniform(*tmem_slot);
+
+    // neighbours share a tile of W: it is read from memory once
+    const int tile = blockIdx.x / CL, rank = CL == 1 ? 0 : blockIdx.x % CL, tok_tiles = (N + TN - 1) / TN;
+    const int tok0 = tile % tok_tiles * TN, m0 = tile / tok_tiles * 128;
+    const int blocks = (K + FS_BK - 1) / FS_BK, quarter = (blocks + 3) / 4, quarters = (blocks + quarter - 1) / quarter;
+    const int kb0 = CL == 1 ? 0 : min(rank * quarter, blocks), nb = CL == 1 ? blocks : min(quarter, blocks - kb0);
+
+    if (warp < 4) {
+        if (TN == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n");
+        if (warp == 0 && lane == 0) {
+            for (int i = 0; i < nb; i++) {
+                const int s = i % FS_RAW, round = i / FS_RAW;
+                if (round > 0 && !mbar_wait(rempty0 + 8 * s, (round - 1) & 1, err)) break;
+                mbar_expect_tx(rfull0 + 8 * s, FS_RAW_BYTES);
+                tma_load_2d(raw0 + s * FS_RAW_BYTES, &wmap, (kb0 + i) * FS_BK, m0, rfull0 + 8 * s);
+            }
+        } else if (warp == 2 && lane == 0) {
+            pdl_wait();                                        // the planes are the kernel before's
+            for (int i = 0; i < nb; i++) {
+                const int s = i % S::STAGES, round = i / S::STAGES;
+                if (round > 0 && !mbar_wait(empty0 + 8 * s, (round - 1) & 1, err)) break;
+                const uint32_t fb = full0 + 8 * s, dst = stage0 + s * S::STAGE + 3 * FS_W_PLANE;
+                mbar_expect_tx(fb, 3 * S::X_PLANE);
+#pragma unroll
+                for (int p = 0; p < 3; p++) tma_load_2d(dst + p * S::X_PLANE, &xmap, (kb0 + i) * FS_BK, p * N + tok0, fb);
+            }
+        } else if (warp == 1) {
+            // the whole warp walks, one lane issues (umma_f16_warp)
+            constexpr uint32_t idesc = umma_idesc(128, TN);
+            constexpr int WP[6] = {1, 0, 2, 0, 1, 0}, XP[6] = {1, 2, 0, 1, 0, 0};      // planes h m l = 0 1 2
+            auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)); };
+            int s = 0, round = 0;
+            for (int i = 0; i < nb; i++) {
+                const int acc = i & 1;
+                if (i > 1 && !wait(tempty0 + 8 * acc, ((i >> 1) - 1) & 1)) break;
+                if (!wait(full0 + 8 * s, round & 1)) break;
+                tc_fence_after();
+                const uint32_t w_lo = (stage0 + s * S::STAGE) >> 4, x_lo = w_lo + (3 * FS_W_PLANE >> 4), d = tmem_base + acc * TN;
+#pragma unroll
+                for (int p = 0; p < 6; p++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++)
+                        umma_f16_warp(d, fs_desc(w_lo + (WP[p] * FS_W_PLANE >> 4) + 2 * k), fs_desc(x_lo + (XP[p] * S::X_PLANE >> 4) + 2 * k),
+                                      idesc, p > 0 || k > 0);
+                umma_commit_warp(empty0 + 8 * s);
+                umma_commit_warp(tfull0 + 8 * acc);
+                if (++s == S::STAGES) { s = 0; round++; }
+            }
+        }
+        __syncwarp();
+    } else if (warp < 8) {
+        if (TN == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;\n");
+        const int t = tid - 128;
+        for (int i = 0; i < nb; i++) {
+            const int rs = i % FS_RAW, s = i % S::STAGES, round = i / S::STAGES;
+            const bool got = mbar_wait(rfull0 + 8 * rs, (i / FS_RAW) & 1, err);
+            if (!__all_sync(0xffffffffu, got)) break;
+            float4 x[8];
+            const unsigned char* raw = smem + S::STAGES * S::STAGE + rs * FS_RAW_BYTES;
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = *reinterpret_cast<const float4*>(raw + (t + j * 128) * 16);
+            const bool free_ = round == 0 || mbar_wait(empty0 + 8 * s, (round - 1) & 1, err);
+            if (!__all_sync(0xffffffffu, free_)) break;
+            unsigned char* dst = smem + s * S::STAGE;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int row = (t >> 3) + j * 16, c = t & 7;           // four values: half of the row's 16-byte piece c / 2
+                uint2 h, m, l;
+                fs_split4(x[j], h, m, l);
+                unsigned char* p = dst + row * 64 + (((c >> 1) ^ ((row >> 1) & 3)) << 4) + (c & 1) * 8;
+                *reinterpret_cast<uint2*>(p) = h;
+                *reinterpret_cast<uint2*>(p + FS_W_PLANE) = m;
+                *reinterpret_cast<uint2*>(p + 2 * FS_W_PLANE) = l;
+            }
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(full0 + 8 * s);
+                mbar_arrive(rempty0 + 8 * rs);
+            }
+        }
+    } else {
+        if (TN == 256) asm volatile("setmaxnreg.inc.sync.aligned.u32 184;\n");
+        const int q = warp & 3, half = (warp - 8) >> 2, m = m0 + q * 32 + lane;
+        const uint32_t taddr = tmem_base + half * HALF + ((uint32_t)(q * 32) << 16);
+        float sum[HALF];
+#pragma unroll
+        for (int j = 0; j < HALF; j++) sum[j] = 0.0f;
+        float* out = C + (size_t)(tok0 + half * HALF) * ldc + m;
+        const int cols = m < M ? min(HALF, N - tok0 - half * HALF) : 0;        // columns this thread has (0 or less: none)
+        bool ok = true, odd = false;
+        pdl_wait();
+        for (int i = 0; i < nb; i++) {
+            const int acc = i & 1;
+            const bool got = mbar_wait(tfull0 + 8 * acc, (i >> 1) & 1, err);
+            if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+            tc_fence_after();
+            const bool first = CL == 1 ? i % quarter == 0 : i == 0;
+            if (HALF >= 32) {
+#pragma unroll
+                for (int c = 0; c < HALF; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + acc * TN + c, r);
+                    tmem_ld_wait();
+                    if (first) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) sum[(c + j) % HALF] = __uint_as_float(r[j]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) sum[(c + j) % HALF] += __uint_as_float(r[j]);
+                    }
+                }
+            } else {
+                uint32_t r[HALF];
+#pragma unroll
+                for (int c = 0; c < HALF; c += 8) fs_ld8(taddr + acc * TN + c, r + c);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < HALF; j++) sum[j] = first ? __uint_as_float(r[j]) : sum[j] + __uint_as_float(r[j]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty0 + 8 * acc);
+            if (CL == 1 && (i + 1 == nb || (i + 1) % quarter == 0)) {
+                const bool start = i < quarter, last = i + 1 == nb;
+                constexpr int B = HALF < 16 ? HALF : 16;
+                int step = ldc;
+                asm volatile("" : "+r"(step));                  // the addresses are made here, not kept over the loop
+                float* p = out;
+#pragma unroll
+                for (int c = 0; c < HALF; c += B, p += (size_t)B * step) {
+                    float before[B];
+#pragma unroll
+                    for (int j = 0; j < B; j++) before[j] = !start && c + j < cols ? p[(size_t)j * step] : 0.0f;
+#pragma unroll
+                    for (int j = 0; j < B; j++) {
+                        const float v = start ? sum[c + j] : before[j] + sum[c + j];
+                        if (c + j < cols) {
+                            p[(size_t)j * step] = v;
+                            if (last) odd |= !fs_finite(v);
+                        }
+                    }
+                }
+            }
+        }
+        if (CL == 1 && ok && odd) {
+            for (int c = 0; c < cols; c++)
+                if (!fs_finite(out[(size_t)c * ldc]))
+                    out[(size_t)c * ldc] = fs_plain_chain(A + (size_t)(tok0 + half * HALF + c) * K, W + (size_t)m * K, K);
+        }
+        if (CL > 1) {
+            // every product and copy of this block is done: its sums go where the stages lay, a row of 128 for every column
+            float* ex = reinterpret_cast<float*>(smem);
+#pragma unroll
+            for (int j = 0; j < HALF; j++) ex[(half * HALF + j) * 128 + q * 32 + lane] = sum[j];
+        }
+    }
+    if (CL > 1) {
+        __syncwarp();
+        fs_cluster_sync();
+        if (warp >= 8) {
+            constexpr int MINE = TN / CL;                       // columns this block adds up
+            const int r = tid & 127, m = m0 + r, c0 = rank * MINE;
+            for (int c = (tid - 256) >> 7; c < MINE; c += 2) {
+                const int n = tok0 + c0 + c;
+                float v = 0.0f;
+                for (int b = 0; b < quarters; b++) {
+                    const float x = fs_ld_cluster(stage0 + ((c0 + c) * 128 + r) * 4, b);
+                    v = b == 0 ? x : v + x;
+                }
+                if (n < N && m < M) {
+                    if (!fs_finite(v)) v = fs_plain_chain(A + (size_t)n * K, W + (size_t)m * K, K);
+                    C[(size_t)n * ldc + m] = v;
+                }
+            }
+        }
+        __syncwarp();
+        fs_cluster_sync();                                      // nobody leaves while its sums are read
+    }
+    // common exit: every role comes here, also after a wait that ran out; then the tensor memory is given back
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, S::TMEM);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ host side
+static int fs_map(const void* base, CUtensorMapDataType type, int item, long long rows, int cols, int box_cols, int box_rows,
+                  CUtensorMapSwizzle swizzle, CUtensorMap* out) {
+    EncodeTiled enc = encode_fn();
+    if (!enc) return -6;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * item};
+    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, estr[2] = {1u, 1u};
+    return enc(out, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -6;
+}
+
+template <int TN, int CL>
+static int fs_launch(const CUtensorMap& wmap, const float* A, const float* W, float* C, const bf16* planes, int N, int M, int K, int Kp,
+                     int ldc, int* err, cudaStream_t st) {
+    CUtensorMap xmap;
+    int rc = fs_map(planes, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 3LL * N, Kp, FS_BK, TN, CU_TENSOR_MAP_SWIZZLE_64B, &xmap);
+    if (rc) return rc;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc5_kernel<TN, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, FsShape<TN>::SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const long long grid = (long long)((N + TN - 1) / TN) * ((M + 127) / 128) * CL;
+    if (grid > 0x7fffffffLL) return -2;
+    cudaError_t e = mb_launch_cluster(mb_pdl, CL, gemm_f32_tc5_kernel<TN, CL>, dim3((unsigned)grid), dim3(FS_THREADS), FsShape<TN>::SMEM,
+                                      st, wmap, xmap, A, W, C, N, M, K, ldc, err);
+    if (e != cudaSuccess) return (int)e;
+    MB_LAUNCH_CHECK();
+    return 0;
+}
+
+// The tile: rows of A a block, and whether a cluster shares K.  Cost of a choice = rounds of blocks x (stages x time of a stage +
+// what a block costs beside them), both as measured (one tile size alone on 2,048 and 8,192 k; the sums of the quarters through C
+// are in it).  A stage takes as long with 16 rows of A as with 128: its twelve instructions wait for each other; with 256 it is
+// bound by the planes that come in from the L2.  us, 128 alone / 128 in fours / 256 alone / 256 in fours: 509 x 16384 x 2048 283 /
+// 362 / 243 / 275, 509 x 2048 x 2048 75 / 53 / 102 / 41, 509 x 2048 x 8192 237 / 134 / 321 / 102, 300 x 16384 x 2048 213 / 274 /
+// 223 / 271; 64 rows x 2048 x 2048 (32 in fours) 24, one row (16 in fours) 22.
+static void fs_choose(int N, int M, int K, int* tn, int* cl) {
+    static const int TNS[5] = {16, 32, 64, 128, 256};
+    static const int STAGE_NS[5][2] = {{883, 883}, {885, 885}, {890, 890}, {845, 850}, {1140, 1256}};
+    static const int BLOCK_NS[5][2] = {{2000, 3500}, {3000, 4000}, {4000, 6000}, {16000, 8000}, {36000, 16000}};
+    const long long blocks = (K + FS_BK - 1) / FS_BK, quarter = (blocks + 3) / 4, rows = (M + 127) / 128;
+    long long best = -1;
+    for (int i = 0; i < 5; i++)
+        for (int c = 0; c < 2; c++) {
+            const long long units = rows * ((N + TNS[i] - 1) / TNS[i]), slots = c ? 36 : 148;          // tiles the device holds at once
+            const long long cost = (units + slots - 1) / slots * ((c ? quarter : blocks) * STAGE_NS[i][c] + BLOCK_NS[i][c]);
+            if (best < 0 || cost < best) { best = cost; *tn = TNS[i]; *cl = c ? 4 : 1; }
+        }
+}
+
+MB_API int mb_gemm_f32_tc5_supports(const void* W, int M, int K) {
+    return K % 4 == 0 && K >= 128 && M >= 64 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+}
+
+// planes: 3 x N x (K rounded up to 8) bf16, working memory.  rows of C are ldc floats apart.  tile (16, 32, 64, 128 or 256 rows of A
+// a block) and cluster (1 or 4 blocks share K): 0 leaves the choice to the sizes; the result is the same.
+MB_API int mb_gemm_f32_tc5(const float* A, const float* W, float* C, bf16* planes, int N, int M, int K, int ldc, int tile, int cluster,
+                           int* err, cudaStream_t st) {
+    if (N == 0 || M == 0) return 0;
+    if (ldc < M || !mb_gemm_f32_tc5_supports(W, M, K) || (reinterpret_cast<uintptr_t>(planes) & 15)) return -2;
+    const int Kp = (K + 7) / 8 * 8;
+    int tn, cl;
+    fs_choose(N, M, K, &tn, &cl);
+    if (tile) tn = tile;
+    if (cluster) cl = cluster;
+    CUtensorMap wmap;
+    int rc = fs_map(W, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, M, K, FS_BK, 128, CU_TENSOR_MAP_SWIZZLE_NONE, &wmap);
+    if (rc) return rc;
+    const size_t quads = (size_t)N * (Kp / 4);
+    const unsigned grid = (unsigned)((quads + 255) / 256 < 2368 ? (quads + 255) / 256 : 2368);
+    if ((reinterpret_cast<uintptr_t>(A) & 15) == 0) split_rows_kernel<true><<<grid, 256, 0, st>>>(A, planes, N, K, Kp);
+    else split_rows_kernel<false><<<grid, 256, 0, st>>>(A, planes, N, K, Kp);
+    MB_LAUNCH_CHECK();
+#define FS_CASE(TN)                                                                                      \
+    if (tn == TN) return cl == 1 ? fs_launch<TN, 1>(wmap, A, W, C, planes, N, M, K, Kp, ldc, err, st)   \
+                                 : fs_launch<TN, 4>(wmap, A, W, C, planes, N, M, K, Kp, ldc, err, st);
+    FS_CASE(16) FS_CASE(32) FS_CASE(64) FS_CASE(128) FS_CASE(256)
+#undef FS_CASE
+    return -2;
+}

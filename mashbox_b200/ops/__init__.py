@@ -83,7 +83,7 @@ def scratch_generation():
 # set through set_pdl(); the engine's option "pdl" turns it on.
 PDL = {"on": False}
 _PDL_SETTERS = {"gemm_stream": "mb_gemm_stream_set_pdl", "elementwise": "mb_elementwise_set_pdl",
-                "attention_tma": "mb_attn_tma_set_pdl"}
+                "attention_tma": "mb_attn_tma_set_pdl", "gemm_f32_tc5": "mb_gemm_f32_tc5_set_pdl"}
 _pdl_applied = {}
 
 
@@ -806,14 +806,18 @@ def moe_combine(y, wts, out, shared=None, gate=None):
 
 
 def linear(a, w, out=None, out_dtype=None):
-    """a (N, K) @ w (M, K)^T -> (N, M).  float32: the package's own fixed-order FFMA kernel (no TF32, no tensor
-    cores).  bfloat16: cuBLAS with float accumulation; out_dtype float32 keeps the accumulator's precision."""
+    """a (N, K) @ w (M, K)^T -> (N, M).  float32: the package's own products of fixed order, true 32-bit (no TF32): on the
+    tensor cores in exact bf16 parts, on the FMA units where w is small or not aligned (by w alone: a row's result does
+    not depend on the number of rows).  bfloat16: cuBLAS with float accumulation; out_dtype float32 keeps the accumulator's
+    precision."""
     _cuda(a, w)
     N, K = a.shape
     M = w.shape[0]
     if a.dtype == torch.float32:
         if out is None:
             out = torch.empty((N, M), dtype=torch.float32, device=a.device)
+        if f32_split_supports(w):
+            return linear_f32_split(a, w, out)
         f = _fn("gemm_f32", "mb_gemm_f32", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
         _check(f(_p(a), _p(w), _p(out), N, M, K, out.stride(0) if N > 1 else M, _stream()), "gemm_f32")
         return out
@@ -844,6 +848,31 @@ def linear(a, w, out=None, out_dtype=None):
     if out is not None:
         return torch.mm(a, w.t(), out=out)
     return torch.mm(a, w.t())
+
+
+def f32_split_supports(w):
+    """the float32 product on the tensor cores (gemm_f32_tc5.cu): by the matrix alone, so that the rows of a step change no bit"""
+    M, K = w.shape
+    return K % 4 == 0 and K >= 128 and M >= 64 and w.data_ptr() % 16 == 0
+
+
+F32_SPLIT_PLANE = 1 << 26          # values of a plane of a's bf16 parts (three planes, 6 bytes a value): more rows go in slabs
+
+
+def linear_f32_split(a, w, out, tile=0, cluster=0):
+    """a (N, K) @ w (M, K)^T -> out (N, M), float32 on the tensor cores.  tile, cluster: rows of a a block takes (16, 32, 64, 128,
+    256) and the blocks that share K (1, 4); 0 leaves the choice to the sizes, and none changes the result."""
+    _cuda(a, w, out)
+    N, K = a.shape
+    M, Kp = w.shape[0], (K + 7) // 8 * 8
+    most = max(256, F32_SPLIT_PLANE // Kp)
+    planes = torch.empty((3 * min(N, most), Kp), dtype=torch.bfloat16, device=a.device)
+    f = _fn("gemm_f32_tc5", "mb_gemm_f32_tc5", [c_void_p] * 4 + [c_int] * 6 + [c_void_p] * 2)
+    for lo in range(0, N, most):
+        n = min(N, lo + most) - lo
+        _check(f(_p(a) + lo * K * 4, _p(w), _p(out) + lo * out.stride(0) * 4, _p(planes), n, M, K, out.stride(0) if N > 1 else M,
+                 int(tile), int(cluster), _p(error_word(a.device)), _stream()), "gemm_f32_tc5")
+    return out
 
 
 def linear_groups(a, w, out):

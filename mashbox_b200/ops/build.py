@@ -26,6 +26,7 @@ HEADERS = ["common.cuh", "attention_common.cuh", "tcgen05.cuh"]
 LIBRARIES = {            # library name -> (source file, extra compiler flags)
     "elementwise": ("elementwise.cu", []),
     "gemm_f32": ("gemm_f32.cu", []),
+    "gemm_f32_tc5": ("gemm_f32_tc5.cu", []),                           # the same product on the tensor cores, in bf16 parts
     "gemm_tc5": ("gemm_tc5.cu", []),
     "gemm_experts": ("gemm_experts.cu", []),                           # routed experts, weights on the M side
     "gemm_stream": ("gemm_stream.cu", []),
