@@ -8,8 +8,8 @@
 // first, the two that carry the result last) and is then added, rounded to nearest, to a sum in registers.  Measured against
 // 64 bits this is nearer than one chain of fused multiply-adds over k (gemm_f32.cu): relative error 0.8e-7 / 1.1e-7 / 1.7e-7 at
 // K 512 / 2,048 / 8,192 on normal values, the chain's 4e-7 / 8e-7 / 16e-7 (tests/test_float32_split_gpu.py).  The FMA units' product
-// at the same size and this one: 509 x 16384 x 2048 684 -> 243 us, 509 x 2048 x 8192 494 -> 102, 1 x 2048 x 8192
-// 405 -> 65; one row of a head of 128,256 alone is slower (333 -> 415).
+// at the same size and this one: 509 x 16384 x 2048 683 -> 241 us, 509 x 2048 x 8192 491 -> 98, 509 x 2048 x 2048 127 -> 41, one
+// row x 2048 x 2048 88 -> 21, one row of a head of 128,256 333 -> 293.
 //
 // An output is the same operations in the same order however many rows a call has: blocks of 32 k in ascending order
 // within a quarter of K, the quarters' sums in ascending order.  Tiles, and whether one block or a cluster of four goes
@@ -365,19 +365,20 @@ static int fs_launch(const CUtensorMap& wmap, const float* A, const float* W, fl
 
 // The tile: rows of A a block, and whether a cluster shares K.  Cost of a choice = rounds of blocks x (stages x time of a stage +
 // what a block costs beside them), both as measured (one tile size alone on 2,048 and 8,192 k; the sums of the quarters through C
-// are in it).  A stage takes as long with 16 rows of A as with 128: its twelve instructions wait for each other; with 256 it is
-// bound by the planes that come in from the L2.  us, 128 alone / 128 in fours / 256 alone / 256 in fours: 509 x 16384 x 2048 283 /
-// 362 / 243 / 275, 509 x 2048 x 2048 75 / 53 / 102 / 41, 509 x 2048 x 8192 237 / 134 / 321 / 102, 300 x 16384 x 2048 213 / 274 /
-// 223 / 271; 64 rows x 2048 x 2048 (32 in fours) 24, one row (16 in fours) 22.
+// are in it).  A stage takes almost as long with 16 rows of A as with 128: its twelve instructions wait for each other; with 256 it
+// is bound by the planes that come in from the L2.  us, 64 alone / 128 alone / 128 in fours / 256 alone / 256 in fours: 509 x 16384
+// x 2048 349 / 264 / 344 / 241 / 263, 509 x 2048 x 2048 57 / 71 / 52 / 103 / 41, 509 x 2048 x 8192 190 / 221 / 129 / 315 / 98,
+// 300 x 3072 x 2048 57 / 71 / 71 / 101 / 71, 300 x 16384 x 2048 250 / 198 / 260 / 228 / 258; one row x 2048 x 2048: 16 alone 47, in
+// fours 21.
 static void fs_choose(int N, int M, int K, int* tn, int* cl) {
     static const int TNS[5] = {16, 32, 64, 128, 256};
-    static const int STAGE_NS[5][2] = {{883, 883}, {885, 885}, {890, 890}, {845, 850}, {1140, 1256}};
-    static const int BLOCK_NS[5][2] = {{2000, 3500}, {3000, 4000}, {4000, 6000}, {16000, 8000}, {36000, 16000}};
+    static const int STAGE_NS[5][2] = {{620, 620}, {640, 640}, {680, 680}, {780, 800}, {1110, 1170}};
+    static const int BLOCK_NS[5][2] = {{2000, 6000}, {3000, 6000}, {9000, 7000}, {16000, 9000}, {38000, 17000}};
     const long long blocks = (K + FS_BK - 1) / FS_BK, quarter = (blocks + 3) / 4, rows = (M + 127) / 128;
     long long best = -1;
     for (int i = 0; i < 5; i++)
         for (int c = 0; c < 2; c++) {
-            const long long units = rows * ((N + TNS[i] - 1) / TNS[i]), slots = c ? 36 : 148;          // tiles the device holds at once
+            const long long units = rows * ((N + TNS[i] - 1) / TNS[i]), slots = c ? 35 : 148;          // tiles the device holds at once
             const long long cost = (units + slots - 1) / slots * ((c ? quarter : blocks) * STAGE_NS[i][c] + BLOCK_NS[i][c]);
             if (best < 0 || cost < best) { best = cost; *tn = TNS[i]; *cl = c ? 4 : 1; }
         }
