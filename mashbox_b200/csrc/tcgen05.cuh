@@ -47,15 +47,11 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
                  ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// the same product with the A operand in tensor memory (row = lane, two bf16 per 32-bit column, k ascending)
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
-// The same three for a warp that walks together, one lane of it issuing: operands that are the same in all lanes stay in the
+// The same for a warp that walks together, one lane of it issuing (umma_f16_ts_warp: the A operand in tensor memory, row = lane,
+// two bf16 per 32-bit column, k ascending): operands that are the same in all lanes stay in the
 // uniform registers the instructions read, while in a branch of one lane each is carried over by itself (some 40 to 100 cycles an
 // instruction, as long as the product of a 128 x 64 x 16 tile takes).  The warp's number, counts and addresses have to be the same
 // in all lanes for the compiler too: warp_uniform().
