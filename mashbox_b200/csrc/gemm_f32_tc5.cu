@@ -1,15 +1,23 @@
 // True 32-bit matrix product on the tensor cores: C[n, m] = sum_k A[n, k] * W[m, k], float32 operands and results.
 //
-// Every float32 operand is cut into three bf16 numbers that add up to it exactly, x = h + m + l (h its upper 8 significant
-// bits, m the rest rounded to 8, l what is left), so a product is a sum of exact bf16 products; the six that matter --
-// m m, h l, l h, h m, m h and h h, in this order; m l, l m and l l lie below 2^-24 of the product -- run as tcgen05.mma
-// (kind::f16, float accumulator).  The tensor cores cut off the low bits of what they add to an accumulator instead of
-// rounding it, so an accumulator never grows old: it takes ONE block of 32 k (twelve instructions, the small parts
-// first, the two that carry the result last) and is then added, rounded to nearest, to a sum in registers.  Measured against
-// 64 bits this is nearer than one chain of fused multiply-adds over k (gemm_f32.cu): relative error 0.8e-7 / 1.1e-7 / 1.7e-7 at
-// K 512 / 2,048 / 8,192 on normal values, the chain's 4e-7 / 8e-7 / 16e-7 (tests/test_float32_split_gpu.py).  The FMA units' product
-// at the same size and this one: 509 x 16384 x 2048 683 -> 241 us, 509 x 2048 x 8192 491 -> 98, 509 x 2048 x 2048 127 -> 41, one
-// row x 2048 x 2048 88 -> 21, one row of a head of 128,256 333 -> 293.
+// Every float32 operand, times 2^24, is cut into three bf16 numbers that add up to it exactly, x = h + m + l (h its upper 8
+// significant bits, m the rest rounded to 8, l what is left; the factor keeps the last bit of the smallest subnormal above
+// what a bf16 can hold), so a product is a sum of exact bf16 products.  Eight of the nine run as tcgen05.mma (kind::f16, float
+// accumulator); l l, left out, is at most 2^-32 of the product.  The tensor cores cut off the low bits of what they add to an
+// accumulator instead of rounding it, so h h, which carries the result, has an accumulator of its own that takes ONE block of
+// 32 k (a single product of 16 bits lies in it exactly) and is then added, rounded to nearest, to a sum in registers.  The
+// other seven, together at most 2^-6 of the product, share two accumulators over up to 512 k and are added to that sum, rounded
+// to nearest.  So a result that one product decides is that product rounded once, as a fused multiply-add rounds it,
+// and sums of many are nearer to 64 bits than one chain of fused multiply-adds over k (gemm_f32.cu): relative error 0.8e-7 /
+// 1.0e-7 / 1.6e-7 at K 512 / 2,048 / 8,192 on normal values, the chain's 4e-7 / 8e-7 / 16e-7; measured by the sum of the products'
+// magnitudes the worst element is nearer too, but where two to a few products of one block of 32 decide a result, what h h is cut
+// off by (up to 2^-23) beside the last rounding is some 1.6 times the chain's few roundings (tests/test_float32_split_gpu.py).
+// (With h h in one accumulator with the rest and m l, l m left out, up to 2^-22 of a product was missing; a block was 12 instructions then,
+// not 10, but 256 rows of A fitted: 509 x 2048 x 2048 37 us, now 49.)  Bound by the chain of a stage: 0.74 us with 128 rows of A, 0.58
+// with 2 of its 10 instructions, 0.51 without the cutting besides; more stages of either ring bring nothing.  W's planes in tensor
+// memory, so that the instructions read half as much shared memory, 0.97 (16 instructions).  The FMA units' product at the same size
+// and this one, us: 509 x 16384 x 2048 684 and 251, 509 x 2048 x 8192 491 and 126, 509 x 2048 x 2048 123 and 49, one row x 2048 x
+// 2048 97 and 17.
 //
 // An output is the same operations in the same order however many rows a call has: blocks of 32 k in ascending order
 // within a quarter of K, the quarters' sums in ascending order.  Tiles, and whether one block or a cluster of four goes
@@ -36,17 +44,21 @@ MB_PDL_SWITCH(mb_gemm_f32_tc5_set_pdl)              // the product starts, and b
 #define FS_RAW_BYTES (128 * FS_BK * 4)
 #define FS_W_PLANE (128 * FS_BK * 2)
 #define FS_THREADS 512
+#define FS_PERIOD 16                               // blocks of 32 k that the accumulators of the small parts take at most
+#define FS_UP 16777216.0f                          // 2^24: what operands are multiplied by before they are cut
+#define FS_DOWN 3.5527136788005009e-15f            // 2^-48: what sums are multiplied by
 
 template <int TN> struct FsShape {
     static constexpr int X_PLANE = TN * FS_BK * 2;
     static constexpr int STAGE = 3 * FS_W_PLANE + 3 * X_PLANE;
-    static constexpr int STAGES = TN == 256 ? 2 : TN == 128 ? 3 : 4;
-    static constexpr int TMEM = 2 * TN < 32 ? 32 : 2 * TN;
+    static constexpr int STAGES = TN == 128 ? 3 : 4;
+    static constexpr int TMEM = 4 * TN;                        // two accumulators of h h in turn, two side by side of the rest
     static constexpr int SMEM = 1024 + STAGES * STAGE + FS_RAW * FS_RAW_BYTES + 256;
 };
 
-// four floats -> their three bf16 parts, two to a word.  h is cut off (never rounded up to infinity), m is rounded, l is exact.
-__device__ __forceinline__ void fs_split4(const float4 x, uint2& h, uint2& m, uint2& l) {
+// four floats -> the three bf16 parts of 2^24 times each, two to a word.  h is cut off, m is rounded, l is exact.
+__device__ __forceinline__ void fs_split4(const float4 v, uint2& h, uint2& m, uint2& l) {
+    const float4 x = make_float4(v.x * FS_UP, v.y * FS_UP, v.z * FS_UP, v.w * FS_UP);
     const uint32_t a = __float_as_uint(x.x), b = __float_as_uint(x.y), c = __float_as_uint(x.z), d = __float_as_uint(x.w);
     h.x = __byte_perm(a, b, 0x7632);
     h.y = __byte_perm(c, d, 0x7632);
@@ -93,6 +105,45 @@ __device__ __forceinline__ void fs_ld8(uint32_t taddr, uint32_t* r) {
                  : "r"(taddr) : "memory");
 }
 
+// sum += (first: =) the HALF columns of an accumulator from taddr on
+template <int HALF> __device__ __forceinline__ void fs_add(uint32_t taddr, bool first, float (&sum)[HALF]) {
+    constexpr int B = HALF < 32 ? HALF : 32;
+#pragma unroll
+    for (int c = 0; c < HALF; c += B) {
+        uint32_t r[32];
+        if (B == 32) tmem_ld32(taddr + c, r);
+        else {
+#pragma unroll
+            for (int j = 0; j < B; j += 8) fs_ld8(taddr + c + j, r + j);
+        }
+        tmem_ld_wait();
+        if (first) {
+#pragma unroll
+            for (int j = 0; j < B; j++) sum[c + j] = __uint_as_float(r[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < B; j++) sum[c + j] += __uint_as_float(r[j]);
+        }
+    }
+}
+
+// sum += the two accumulators of the small parts, TN columns apart
+template <int HALF, int TN> __device__ __forceinline__ void fs_add_small(uint32_t taddr, float (&sum)[HALF]) {
+    constexpr int B = HALF < 16 ? HALF : 16;
+#pragma unroll
+    for (int c = 0; c < HALF; c += B) {
+        uint32_t r[B], t[B];
+#pragma unroll
+        for (int j = 0; j < B; j += 8) {
+            fs_ld8(taddr + c + j, r + j);
+            fs_ld8(taddr + TN + c + j, t + j);
+        }
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < B; j++) sum[c + j] += __uint_as_float(r[j]) + __uint_as_float(t[j]);
+    }
+}
+
 __device__ __noinline__ float fs_plain_chain(const float* a, const float* w, int K) {
     float s = 0.0f;
     for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
@@ -125,13 +176,16 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::STAGES * S::STAGE + FS_RAW * FS_RAW_BYTES);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * S::STAGES, rfull0 = empty0 + 8 * S::STAGES,
-                   rempty0 = rfull0 + 8 * FS_RAW, tfull0 = rempty0 + 8 * FS_RAW, tempty0 = tfull0 + 16;
+                   rempty0 = rfull0 + 8 * FS_RAW, tfull0 = rempty0 + 8 * FS_RAW, tempty0 = tfull0 + 16, sfull = tempty0 + 16,
+                   sempty = sfull + 8;
     const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
 
     if (tid == 0) {
         for (int s = 0; s < S::STAGES; s++) { mbar_init(full0 + 8 * s, 5); mbar_init(empty0 + 8 * s, 1); }
         for (int s = 0; s < FS_RAW; s++) { mbar_init(rfull0 + 8 * s, 1); mbar_init(rempty0 + 8 * s, 4); }
         for (int a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 8); }
+        mbar_init(sfull, 1);
+        mbar_init(sempty, 8);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
@@ -151,7 +205,6 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     const int kb0 = CL == 1 ? 0 : min(rank * quarter, blocks), nb = CL == 1 ? blocks : min(quarter, blocks - kb0);
 
     if (warp < 4) {
-        if (TN == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n");
         if (warp == 0 && lane == 0) {
             for (int i = 0; i < nb; i++) {
                 const int s = i % FS_RAW, round = i / FS_RAW;
@@ -171,51 +224,62 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             }
         } else if (warp == 1) {
             // the whole warp walks, one lane issues (umma_f16_warp)
-            constexpr uint32_t idesc = umma_idesc(128, TN);
-            constexpr int WP[6] = {1, 0, 2, 0, 1, 0}, XP[6] = {1, 2, 0, 1, 0, 0};      // planes h m l = 0 1 2
+            constexpr uint32_t one = umma_idesc(128, TN), two = umma_idesc(128, 2 * TN);
             auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)); };
-            int s = 0, round = 0;
+            int s = 0, round = 0, at = 0, periods = 0;          // at: blocks into the quarter; periods of the small parts begun
+            const uint32_t small = tmem_base + 2 * TN;
             for (int i = 0; i < nb; i++) {
                 const int acc = i & 1;
                 if (i > 1 && !wait(tempty0 + 8 * acc, ((i >> 1) - 1) & 1)) break;
                 if (!wait(full0 + 8 * s, round & 1)) break;
                 tc_fence_after();
-                const uint32_t w_lo = (stage0 + s * S::STAGE) >> 4, x_lo = w_lo + (3 * FS_W_PLANE >> 4), d = tmem_base + acc * TN;
+                // planes of 128 rows of W; planes of TN rows of A, one below the other: h m and m l are tiles of 2 TN rows
+                const uint32_t w = (stage0 + s * S::STAGE) >> 4, x = w + (3 * FS_W_PLANE >> 4);
+                constexpr uint32_t WP = FS_W_PLANE >> 4, XP = S::X_PLANE >> 4;
 #pragma unroll
-                for (int p = 0; p < 6; p++)
-#pragma unroll
-                    for (int k = 0; k < 2; k++)
-                        umma_f16_warp(d, fs_desc(w_lo + (WP[p] * FS_W_PLANE >> 4) + 2 * k), fs_desc(x_lo + (XP[p] * S::X_PLANE >> 4) + 2 * k),
-                                      idesc, p > 0 || k > 0);
-                umma_commit_warp(empty0 + 8 * s);
+                for (int k = 0; k < 4; k += 2) umma_f16_warp(tmem_base + acc * TN, fs_desc(w + k), fs_desc(x + k), one, k > 0);
                 umma_commit_warp(tfull0 + 8 * acc);
+                const bool fresh = at % FS_PERIOD == 0;
+                if (fresh) {
+                    if (periods > 0 && !wait(sempty, (periods - 1) & 1)) break;
+                    tc_fence_after();
+                    periods++;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k += 2) {
+                    umma_f16_warp(small, fs_desc(w + WP + k), fs_desc(x + k), two, k > 0 || !fresh);            // m h, m m
+                    umma_f16_warp(small, fs_desc(w + k), fs_desc(x + XP + k), two, 1u);                         // h m, h l
+                    umma_f16_warp(small, fs_desc(w + 2 * WP + k), fs_desc(x + k), two, 1u);                     // l h, l m
+                    umma_f16_warp(small, fs_desc(w + WP + k), fs_desc(x + 2 * XP + k), one, 1u);                // m l
+                }
+                umma_commit_warp(empty0 + 8 * s);
+                at++;
+                if (at % FS_PERIOD == 0 || at == quarter || i + 1 == nb) umma_commit_warp(sfull);
+                if (at == quarter) at = 0;
                 if (++s == S::STAGES) { s = 0; round++; }
             }
         }
         __syncwarp();
     } else if (warp < 8) {
-        if (TN == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;\n");
         const int t = tid - 128;
         for (int i = 0; i < nb; i++) {
             const int rs = i % FS_RAW, s = i % S::STAGES, round = i / S::STAGES;
             const bool got = mbar_wait(rfull0 + 8 * rs, (i / FS_RAW) & 1, err);
             if (!__all_sync(0xffffffffu, got)) break;
-            float4 x[8];
+            uint2 h[8], m[8], l[8];                             // cut before the stage they go to is waited for
             const unsigned char* raw = smem + S::STAGES * S::STAGE + rs * FS_RAW_BYTES;
 #pragma unroll
-            for (int j = 0; j < 8; j++) x[j] = *reinterpret_cast<const float4*>(raw + (t + j * 128) * 16);
+            for (int j = 0; j < 8; j++) fs_split4(*reinterpret_cast<const float4*>(raw + (t + j * 128) * 16), h[j], m[j], l[j]);
             const bool free_ = round == 0 || mbar_wait(empty0 + 8 * s, (round - 1) & 1, err);
             if (!__all_sync(0xffffffffu, free_)) break;
             unsigned char* dst = smem + s * S::STAGE;
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const int row = (t >> 3) + j * 16, c = t & 7;           // four values: half of the row's 16-byte piece c / 2
-                uint2 h, m, l;
-                fs_split4(x[j], h, m, l);
                 unsigned char* p = dst + row * 64 + (((c >> 1) ^ ((row >> 1) & 3)) << 4) + (c & 1) * 8;
-                *reinterpret_cast<uint2*>(p) = h;
-                *reinterpret_cast<uint2*>(p + FS_W_PLANE) = m;
-                *reinterpret_cast<uint2*>(p + 2 * FS_W_PLANE) = l;
+                *reinterpret_cast<uint2*>(p) = h[j];
+                *reinterpret_cast<uint2*>(p + FS_W_PLANE) = m[j];
+                *reinterpret_cast<uint2*>(p + 2 * FS_W_PLANE) = l[j];
             }
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             __syncwarp();
@@ -225,7 +289,6 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             }
         }
     } else {
-        if (TN == 256) asm volatile("setmaxnreg.inc.sync.aligned.u32 184;\n");
         const int q = warp & 3, half = (warp - 8) >> 2, m = m0 + q * 32 + lane;
         const uint32_t taddr = tmem_base + half * HALF + ((uint32_t)(q * 32) << 16);
         float sum[HALF];
@@ -234,41 +297,36 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         float* out = C + (size_t)(tok0 + half * HALF) * ldc + m;
         const int cols = m < M ? min(HALF, N - tok0 - half * HALF) : 0;        // columns this thread has (0 or less: none)
         bool ok = true, odd = false;
+        int at = 0, periods = 0;                                // as the products count them
         pdl_wait();
         for (int i = 0; i < nb; i++) {
             const int acc = i & 1;
-            const bool got = mbar_wait(tfull0 + 8 * acc, (i >> 1) & 1, err);
+            bool got = mbar_wait(tfull0 + 8 * acc, (i >> 1) & 1, err);
             if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
             tc_fence_after();
-            const bool first = CL == 1 ? i % quarter == 0 : i == 0;
-            if (HALF >= 32) {
-#pragma unroll
-                for (int c = 0; c < HALF; c += 32) {
-                    uint32_t r[32];
-                    tmem_ld32(taddr + acc * TN + c, r);
-                    tmem_ld_wait();
-                    if (first) {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) sum[(c + j) % HALF] = __uint_as_float(r[j]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) sum[(c + j) % HALF] += __uint_as_float(r[j]);
-                    }
-                }
-            } else {
-                uint32_t r[HALF];
-#pragma unroll
-                for (int c = 0; c < HALF; c += 8) fs_ld8(taddr + acc * TN + c, r + c);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < HALF; j++) sum[j] = first ? __uint_as_float(r[j]) : sum[j] + __uint_as_float(r[j]);
-            }
+            fs_add<HALF>(taddr + acc * TN, at == 0, sum);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty0 + 8 * acc);
-            if (CL == 1 && (i + 1 == nb || (i + 1) % quarter == 0)) {
+            at++;
+            const bool ends = at == quarter || i + 1 == nb;
+            if (ends || at % FS_PERIOD == 0) {
+                got = mbar_wait(sfull, periods & 1, err);
+                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+                periods++;
+                tc_fence_after();
+                fs_add_small<HALF, TN>(taddr + 2 * TN, sum);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sempty);
+            }
+            if (ends) {
+#pragma unroll
+                for (int j = 0; j < HALF; j++) sum[j] *= FS_DOWN;
+            }
+            if (CL == 1 && ends) {
                 const bool start = i < quarter, last = i + 1 == nb;
-                constexpr int B = HALF < 16 ? HALF : 16;
+                constexpr int B = 8;
                 int step = ldc;
                 asm volatile("" : "+r"(step));                  // the addresses are made here, not kept over the loop
                 float* p = out;
@@ -287,6 +345,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                     }
                 }
             }
+            if (at == quarter) at = 0;
         }
         if (CL == 1 && ok && odd) {
             for (int c = 0; c < cols; c++)
@@ -365,18 +424,16 @@ static int fs_launch(const CUtensorMap& wmap, const float* A, const float* W, fl
 
 // The tile: rows of A a block, and whether a cluster shares K.  Cost of a choice = rounds of blocks x (stages x time of a stage +
 // what a block costs beside them), both as measured (one tile size alone on 2,048 and 8,192 k; the sums of the quarters through C
-// are in it).  A stage takes almost as long with 16 rows of A as with 128: its twelve instructions wait for each other; with 256 it
-// is bound by the planes that come in from the L2.  us, 64 alone / 128 alone / 128 in fours / 256 alone / 256 in fours: 509 x 16384
-// x 2048 349 / 264 / 344 / 241 / 263, 509 x 2048 x 2048 57 / 71 / 52 / 103 / 41, 509 x 2048 x 8192 190 / 221 / 129 / 315 / 98,
-// 300 x 3072 x 2048 57 / 71 / 71 / 101 / 71, 300 x 16384 x 2048 250 / 198 / 260 / 228 / 258; one row x 2048 x 2048: 16 alone 47, in
-// fours 21.
+// are in it).  us, 64 alone / 128 alone / 128 in fours: 509 x 16384 x 2048 350 / 258 / 357, 509 x 2048 x 2048 55 / 67 / 50, 509 x 2048 x
+// 8192 189 / 218 / 128, 509 x 3072 x 2048 102 / 67 / 72, 300 x 16384 x 2048 247 / 194 / 270, 64 x 2048 x 256 14 / 20 / 13 (32 in fours 8.4);
+// one row x 2048 x 2048: 16 alone 45, in fours 17.
 static void fs_choose(int N, int M, int K, int* tn, int* cl) {
-    static const int TNS[5] = {16, 32, 64, 128, 256};
-    static const int STAGE_NS[5][2] = {{620, 620}, {640, 640}, {680, 680}, {780, 800}, {1110, 1170}};
-    static const int BLOCK_NS[5][2] = {{2000, 6000}, {3000, 6000}, {9000, 7000}, {16000, 9000}, {38000, 17000}};
+    static const int TNS[4] = {16, 32, 64, 128};
+    static const int STAGE_NS[4][2] = {{575, 575}, {630, 600}, {680, 650}, {740, 760}};
+    static const int BLOCK_NS[4][2] = {{4000, 6000}, {5000, 6000}, {9000, 7000}, {16000, 10000}};
     const long long blocks = (K + FS_BK - 1) / FS_BK, quarter = (blocks + 3) / 4, rows = (M + 127) / 128;
     long long best = -1;
-    for (int i = 0; i < 5; i++)
+    for (int i = 0; i < 4; i++)
         for (int c = 0; c < 2; c++) {
             const long long units = rows * ((N + TNS[i] - 1) / TNS[i]), slots = c ? 35 : 148;          // tiles the device holds at once
             const long long cost = (units + slots - 1) / slots * ((c ? quarter : blocks) * STAGE_NS[i][c] + BLOCK_NS[i][c]);
@@ -388,8 +445,8 @@ MB_API int mb_gemm_f32_tc5_supports(const void* W, int M, int K) {
     return K % 4 == 0 && K >= 128 && M >= 64 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
 }
 
-// planes: 3 x N x (K rounded up to 8) bf16, working memory.  rows of C are ldc floats apart.  tile (16, 32, 64, 128 or 256 rows of A
-// a block) and cluster (1 or 4 blocks share K): 0 leaves the choice to the sizes; the result is the same.
+// planes: 3 x N x (K rounded up to 8) bf16, working memory.  rows of C are ldc floats apart.  tile (16, 32, 64 or 128 rows of A
+// a block; more: 128) and cluster (1 or 4 blocks share K): 0 leaves the choice to the sizes; the result is the same.
 MB_API int mb_gemm_f32_tc5(const float* A, const float* W, float* C, bf16* planes, int N, int M, int K, int ldc, int tile, int cluster,
                            int* err, cudaStream_t st) {
     if (N == 0 || M == 0) return 0;
@@ -397,7 +454,7 @@ MB_API int mb_gemm_f32_tc5(const float* A, const float* W, float* C, bf16* plane
     const int Kp = (K + 7) / 8 * 8;
     int tn, cl;
     fs_choose(N, M, K, &tn, &cl);
-    if (tile) tn = tile;
+    if (tile) tn = tile < 128 ? tile : 128;
     if (cluster) cl = cluster;
     CUtensorMap wmap;
     int rc = fs_map(W, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, M, K, FS_BK, 128, CU_TENSOR_MAP_SWIZZLE_NONE, &wmap);
@@ -410,7 +467,7 @@ MB_API int mb_gemm_f32_tc5(const float* A, const float* W, float* C, bf16* plane
 #define FS_CASE(TN)                                                                                      \
     if (tn == TN) return cl == 1 ? fs_launch<TN, 1>(wmap, A, W, C, planes, N, M, K, Kp, ldc, err, st)   \
                                  : fs_launch<TN, 4>(wmap, A, W, C, planes, N, M, K, Kp, ldc, err, st);
-    FS_CASE(16) FS_CASE(32) FS_CASE(64) FS_CASE(128) FS_CASE(256)
+    FS_CASE(16) FS_CASE(32) FS_CASE(64) FS_CASE(128)
 #undef FS_CASE
     return -2;
 }

@@ -806,9 +806,10 @@ def moe_combine(y, wts, out, shared=None, gate=None):
 
 
 def linear(a, w, out=None, out_dtype=None):
-    """a (N, K) @ w (M, K)^T -> (N, M).  float32: the package's own products of fixed order, true 32-bit (no TF32): on the
-    tensor cores in exact bf16 parts, on the FMA units where w is small or not aligned (by w alone: a row's result does
-    not depend on the number of rows).  bfloat16: cuBLAS with float accumulation; out_dtype float32 keeps the accumulator's
+    """a (N, K) @ w (M, K)^T -> (N, M).  float32: the package's own products of fixed order, no TF32: on the tensor cores in
+    bf16 parts that keep every bit of an operand and all of a product but 2^-32 of it (gemm_f32_tc5.cu says how sums compare
+    with a chain of fused multiply-adds), on the FMA units where w is small or not aligned (by w alone: a row's result does not
+    depend on the number of rows).  bfloat16: cuBLAS with float accumulation; out_dtype float32 keeps the accumulator's
     precision."""
     _cuda(a, w)
     N, K = a.shape
@@ -860,8 +861,8 @@ F32_SPLIT_PLANE = 1 << 26          # values of a plane of a's bf16 parts (three 
 
 
 def linear_f32_split(a, w, out, tile=0, cluster=0):
-    """a (N, K) @ w (M, K)^T -> out (N, M), float32 on the tensor cores.  tile, cluster: rows of a a block takes (16, 32, 64, 128,
-    256) and the blocks that share K (1, 4); 0 leaves the choice to the sizes, and none changes the result."""
+    """a (N, K) @ w (M, K)^T -> out (N, M), float32 on the tensor cores.  tile, cluster: rows of a a block takes (16, 32, 64, 128;
+    more is 128) and the blocks that share K (1, 4); 0 leaves the choice to the sizes, and none changes the result."""
     _cuda(a, w, out)
     N, K = a.shape
     M, Kp = w.shape[0], (K + 7) // 8 * 8

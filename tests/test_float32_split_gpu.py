@@ -86,3 +86,84 @@ def test_rows_in_slabs(monkeypatch):
     whole = K.linear(a, w)
     monkeypatch.setattr(K, "F32_SPLIT_PLANE", 1)
     assert torch.equal(K.linear(a, w), whole)
+
+
+def worst(x, exact):
+    """the largest error of an element over that element, where the result is a normal number"""
+    at = exact.abs() >= 2.0 ** -125
+    return float(((x.double() - exact).abs()[at] / exact.abs()[at]).max())
+
+
+def of_bits(n, g):
+    """values of [1, 2) with all their bits drawn"""
+    return (0x3f800000 + torch.randint(0, 1 << 23, (n,), generator=g, dtype=torch.int32)).view(torch.float32).to(G.DEV)
+
+
+# Where few products decide a result: rows that are one value throughout (every product of a result has the same parts left over;
+# 0x3f80ff80 is the worst of all mantissas for parts that are left out), rows of one value and zeros, rows of one value among others
+# that are 2^-34 of it together.  The chain rounds a product once, 2^-24; the bar beside its worst element is that and the parts of 2^-7, which an
+# accumulator may cut off at 2^-23 of them.
+@pytest.mark.parametrize("kind", ["constant", "the worst constant", "one-hot", "dominant"])
+@pytest.mark.parametrize("Kd", [128, 512, 2048])
+@pytest.mark.parametrize("tile,cluster", [(0, 0), (64, 1), (64, 4), (256, 1)])
+def test_few_products_are_as_exact_as_in_a_chain(kind, Kd, tile, cluster):
+    K = ops()
+    N, M = 48, 192
+    g = torch.Generator().manual_seed(Kd)
+    if kind == "constant":
+        a, w = of_bits(N, g)[:, None].repeat(1, Kd), of_bits(M, g)[:, None].repeat(1, Kd)
+    elif kind == "the worst constant":
+        x = torch.tensor([0x3f80ff80], dtype=torch.int32).view(torch.float32).to(G.DEV)
+        a, w = x.repeat(N, Kd), x.repeat(M, Kd)
+    else:
+        w = of_bits(M * Kd, g).view(M, Kd)
+        a = torch.zeros(N, Kd, device=G.DEV) if kind == "one-hot" else of_bits(N * Kd, g).view(N, Kd) * 2.0 ** -34 / Kd
+        a[torch.arange(N), torch.randint(0, Kd, (N,), generator=g)] = of_bits(N, g)
+    exact = a.double() @ w.double().T
+    got = K.linear_f32_split(a, w, torch.empty(N, M, device=G.DEV), tile=tile, cluster=cluster)
+    assert worst(got, exact) <= max(worst(chain(a, w), exact), 2.0 ** -24) * (1 + 2.0 ** -6)
+
+
+@pytest.mark.parametrize("kind", ["normal", "positive", "wide", "tiny"])
+@pytest.mark.parametrize("Kd", [128, 512, 2048, 8192, 16384])
+def test_the_worst_element_is_no_further_off_than_a_chains(kind, Kd):
+    """measured by the sum of the products' magnitudes; and sums that many products make, by themselves"""
+    K = ops()
+    a, w = operands(64, 512, Kd, kind, seed=5)
+    exact, size = a.double() @ w.double().T, a.abs().double() @ w.abs().double().T
+    got, old = K.linear(a, w), chain(a, w)
+    assert float(((got - exact).abs() / size).max()) <= float(((old - exact).abs() / size).max())
+    if kind != "wide":
+        assert float((got - exact).norm()) <= max(float((old - exact).norm()), 2.0 ** -24 * float(exact.norm()))
+
+
+@pytest.mark.parametrize("p", [-96, -109, -112, -118, -124, -130, -140, -149])
+@pytest.mark.parametrize("side", ["a", "w", "both"])
+def test_tiny_operands_keep_all_their_bits(p, side):
+    """operands down to the smallest subnormal, beside ones that bring the products back among the normal numbers"""
+    K = ops()
+    N, M, Kd = 24, 70, 256
+    g = torch.Generator().manual_seed(-p)
+    tiny = lambda n: torch.ldexp(of_bits(n, g).double(), torch.tensor(p, device=G.DEV)).float()
+    big = lambda n: of_bits(n, g) * 2.0 ** min(-p, 100)
+    a = (tiny(N * Kd) if side != "w" else big(N * Kd)).view(N, Kd)
+    w = (tiny(M * Kd) if side != "a" else big(M * Kd)).view(M, Kd)
+    a[:, 1::2] *= -1.0
+    exact = a.double() @ w.double().T
+    # the last bit of a result that is itself subnormal; a chain may lose it at every k, the quarters of K here at their ends
+    err = lambda x: float(((x.double() - exact).abs() - 4 * 2.0 ** -149).clamp(min=0).norm() / exact.norm().clamp(min=2.0 ** -149))
+    assert err(K.linear_f32_split(a, w, torch.empty(N, M, device=G.DEV))) <= max(err(chain(a, w)), 2.0 ** -24)
+
+
+@pytest.mark.parametrize("cluster", [1, 4])
+def test_it_is_float32_arithmetic(cluster):
+    """1 + 2^-p is a float32 number down to p = 23: as a sum of two products, and as one operand"""
+    K = ops()
+    w = torch.zeros(64, 128, device=G.DEV)
+    w[:, 0] = w[:, 70] = 1.0
+    a = torch.zeros(48, 128, device=G.DEV)
+    for p in range(24):
+        a[p, 0], a[p, 70] = 1.0, 2.0 ** -p
+        a[24 + p, 0] = 1.0 + 2.0 ** -p
+    out = K.linear_f32_split(a, w, torch.empty(48, 64, device=G.DEV), cluster=cluster)
+    assert torch.equal(out, (a[:, :1] + a[:, 70:71]).expand(48, 64))
