@@ -13,7 +13,7 @@
 // magnitudes the worst element is nearer too, but where two to a few products of one block of 32 decide a result, what h h is cut
 // off by (up to 2^-23) beside the last rounding is some 1.6 times the chain's few roundings (tests/test_float32_split_gpu.py).
 // (With h h in one accumulator with the rest and m l, l m left out, up to 2^-22 of a product was missing; a block was 12 instructions then,
-// not 10, but 256 rows of A fitted: 509 x 2048 x 2048 37 us, now 49.)  Bound by the chain of a stage: 0.74 us with 128 rows of A, 0.58
+// not 10, but 256 rows of A fitted: 509 x 2048 x 2048 37 us, now 49.)  Bound by the chain of a stage: 0.73 us with 128 rows of A, 0.58
 // with 2 of its 10 instructions, 0.51 without the cutting besides; more stages of either ring bring nothing.  W's planes in tensor
 // memory, so that the instructions read half as much shared memory, 0.97 (16 instructions).  The FMA units' product at the same size
 // and this one, us: 509 x 16384 x 2048 684 and 251, 509 x 2048 x 8192 491 and 126, 509 x 2048 x 2048 123 and 49, one row x 2048 x
@@ -28,6 +28,7 @@
 //   warp 2      TMA: the three bf16 planes of TN x 32 values of A (64-byte swizzle), cut by split_rows_kernel beforehand:
 //               they are read once per tile of W, W once per tile of A
 //   warps 4-7   cut a stage of W into its three planes in shared memory, as the instructions want them
+//   warp 3      tells the products' barrier that planes have come
 //   warp 1      one lane issues the products; accumulators of TN columns, two in turn
 //   warps 8-15  add a block's accumulator to the sums in registers (thread = a row of W, half of the columns)
 // A cluster of four blocks takes a quarter of K each where the tiles alone leave the device idle: the sums meet in
@@ -53,7 +54,7 @@ template <int TN> struct FsShape {
     static constexpr int STAGE = 3 * FS_W_PLANE + 3 * X_PLANE;
     static constexpr int STAGES = TN == 128 ? 3 : 4;
     static constexpr int TMEM = 4 * TN;                        // two accumulators of h h in turn, two side by side of the rest
-    static constexpr int SMEM = 1024 + STAGES * STAGE + FS_RAW * FS_RAW_BYTES + 256;
+    static constexpr int SMEM = 1024 + STAGES * STAGE + FS_RAW * FS_RAW_BYTES + 320;
 };
 
 // four floats -> the three bf16 parts of 2^24 times each, two to a word.  h is cut off, m is rounded, l is exact.
@@ -174,17 +175,19 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
     const uint32_t stage0 = smem_u32(smem), raw0 = stage0 + S::STAGES * S::STAGE;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::STAGES * S::STAGE + FS_RAW * FS_RAW_BYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * S::STAGES, rfull0 = empty0 + 8 * S::STAGES,
-                   rempty0 = rfull0 + 8 * FS_RAW, tfull0 = rempty0 + 8 * FS_RAW, tempty0 = tfull0 + 16, sfull = tempty0 + 16,
-                   sempty = sfull + 8;
+                   rempty0 = rfull0 + 8 * FS_RAW, tfull0 = rempty0 + 8 * FS_RAW, sfull = tfull0 + 16, sempty = sfull + 8,
+                   xfull0 = sempty + 8, done = xfull0 + 8 * S::STAGES;
     const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
 
     if (tid == 0) {
-        for (int s = 0; s < S::STAGES; s++) { mbar_init(full0 + 8 * s, 5); mbar_init(empty0 + 8 * s, 1); }
+        // a stage: four warps that cut W, the planes of A, eight warps that have read the accumulator it goes to
+        for (int s = 0; s < S::STAGES; s++) { mbar_init(full0 + 8 * s, 13); mbar_init(xfull0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
         for (int s = 0; s < FS_RAW; s++) { mbar_init(rfull0 + 8 * s, 1); mbar_init(rempty0 + 8 * s, 4); }
-        for (int a = 0; a < 2; a++) { mbar_init(tfull0 + 8 * a, 1); mbar_init(tempty0 + 8 * a, 8); }
+        for (int a = 0; a < 2; a++) mbar_init(tfull0 + 8 * a, 1);
         mbar_init(sfull, 1);
+        mbar_init(done, 1);
         mbar_init(sempty, 8);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -206,21 +209,32 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
 
     if (warp < 4) {
         if (warp == 0 && lane == 0) {
-            for (int i = 0; i < nb; i++) {
+            int i = 0;
+            for (; i < nb; i++) {
                 const int s = i % FS_RAW, round = i / FS_RAW;
                 if (round > 0 && !mbar_wait(rempty0 + 8 * s, (round - 1) & 1, err)) break;
                 mbar_expect_tx(rfull0 + 8 * s, FS_RAW_BYTES);
                 tma_load_2d(raw0 + s * FS_RAW_BYTES, &wmap, (kb0 + i) * FS_BK, m0, rfull0 + 8 * s);
             }
+            copies_landed(rfull0, FS_RAW, i, err);
         } else if (warp == 2 && lane == 0) {
             pdl_wait();                                        // the planes are the kernel before's
-            for (int i = 0; i < nb; i++) {
+            int i = 0;
+            for (; i < nb; i++) {
                 const int s = i % S::STAGES, round = i / S::STAGES;
                 if (round > 0 && !mbar_wait(empty0 + 8 * s, (round - 1) & 1, err)) break;
-                const uint32_t fb = full0 + 8 * s, dst = stage0 + s * S::STAGE + 3 * FS_W_PLANE;
+                const uint32_t fb = xfull0 + 8 * s, dst = stage0 + s * S::STAGE + 3 * FS_W_PLANE;
                 mbar_expect_tx(fb, 3 * S::X_PLANE);
 #pragma unroll
                 for (int p = 0; p < 3; p++) tma_load_2d(dst + p * S::X_PLANE, &xmap, (kb0 + i) * FS_BK, p * N + tok0, fb);
+            }
+            copies_landed(xfull0, S::STAGES, i, err);
+        } else if (warp == 3 && lane == 0) {
+            // the planes of A have a barrier of their own, so that their copies can be waited for by themselves; the products wait on one
+            // barrier a stage, which hears of them from here (with two waits a stage of 16 rows took 0.84 us, not 0.6)
+            for (int i = 0; i < nb; i++) {
+                if (!mbar_wait(xfull0 + 8 * (i % S::STAGES), (i / S::STAGES) & 1, err)) break;
+                mbar_arrive(full0 + 8 * (i % S::STAGES));
             }
         } else if (warp == 1) {
             // the whole warp walks, one lane issues (umma_f16_warp)
@@ -230,7 +244,6 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             const uint32_t small = tmem_base + 2 * TN;
             for (int i = 0; i < nb; i++) {
                 const int acc = i & 1;
-                if (i > 1 && !wait(tempty0 + 8 * acc, ((i >> 1) - 1) & 1)) break;
                 if (!wait(full0 + 8 * s, round & 1)) break;
                 tc_fence_after();
                 // planes of 128 rows of W; planes of TN rows of A, one below the other: h m and m l are tiles of 2 TN rows
@@ -258,6 +271,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 if (at == quarter) at = 0;
                 if (++s == S::STAGES) { s = 0; round++; }
             }
+            products_landed<true>(done, err);
         }
         __syncwarp();
     } else if (warp < 8) {
@@ -298,6 +312,11 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         const int cols = m < M ? min(HALF, N - tok0 - half * HALF) : 0;        // columns this thread has (0 or less: none)
         bool ok = true, odd = false;
         int at = 0, periods = 0;                                // as the products count them
+        // an accumulator that has been read is among the arrivals that the products of the block after the next wait for
+        if (lane == 0) {
+            mbar_arrive(full0);
+            if (nb > 1) mbar_arrive(full0 + 8);
+        }
         pdl_wait();
         for (int i = 0; i < nb; i++) {
             const int acc = i & 1;
@@ -307,7 +326,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             fs_add<HALF>(taddr + acc * TN, at == 0, sum);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(tempty0 + 8 * acc);
+            if (lane == 0 && i + 2 < nb) mbar_arrive(full0 + 8 * ((i + 2) % S::STAGES));
             at++;
             const bool ends = at == quarter || i + 1 == nb;
             if (ends || at % FS_PERIOD == 0) {

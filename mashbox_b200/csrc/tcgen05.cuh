@@ -68,6 +68,18 @@ __device__ __forceinline__ void umma_commit_warp(uint32_t bar) {
     asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
                  ::"r"(bar) : "memory");
 }
+// Before a block leaves, also after a wait that ran out: whatever it has sent for has to have arrived, since its shared and tensor
+// memory go to the next block.  copies_landed: the thread that sent for `sent` stages of a ring whose barriers full0 + 8 s complete by
+// the copies alone.  products_landed: the warp (umma_..._warp) or the thread that issued products; `done` is a barrier of one arrival
+// that nothing else uses.
+__device__ __forceinline__ void copies_landed(uint32_t full0, int stages, int sent, int* err) {
+    for (int i = sent > stages ? sent - stages : 0; i < sent; i++) mbar_wait(full0 + 8 * (i % stages), (i / stages) & 1, err);
+}
+template <bool WARP> __device__ __forceinline__ void products_landed(uint32_t done, int* err) {
+    if (WARP) umma_commit_warp(done);
+    else umma_commit(done);
+    mbar_wait(done, 0, err);
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
