@@ -42,9 +42,9 @@ gemm_experts_kernel(const __grid_constant__ CUtensorMap amap, const __grid_const
     unsigned char* smem = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)GE_STAGES * GE_STAGE_BYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GE_STAGES + 2);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GE_STAGES + 3);
     const uint32_t stage0 = smem_u32(smem), full0 = smem_u32(bars), empty0 = full0 + 8 * GE_STAGES, tfull = empty0 + 8 * GE_STAGES,
-                   tempty = tfull + 8;
+                   tempty = tfull + 8, done = tempty + 8;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     __shared__ int list[GE_LIST];
     __shared__ int listed;
@@ -53,6 +53,7 @@ gemm_experts_kernel(const __grid_constant__ CUtensorMap amap, const __grid_const
         for (int s = 0; s < GE_STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
         mbar_init(tfull, 1);
         mbar_init(tempty, 8);
+        mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
@@ -104,6 +105,7 @@ gemm_experts_kernel(const __grid_constant__ CUtensorMap amap, const __grid_const
                         tma_load_2d(dst + 2 * GE_W_BYTES + b * GE_BOX_BYTES, &amap, kb * GE_BK, x.row0 + b * GE_BOX, fb);
                 }
             }
+            copies_landed(full0, GE_STAGES, it, err);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -133,6 +135,7 @@ gemm_experts_kernel(const __grid_constant__ CUtensorMap amap, const __grid_const
                 umma_commit(tfull);
                 j++;
             }
+            products_landed<false>(done, err);
         }
         __syncwarp();
     } else if (warp >= 4) {
@@ -204,7 +207,7 @@ static int experts_launch(const void* act, const void* W, void* out, int N, int 
     if (rc) return rc;
     rc = matrix_map(W, (long long)(GATED ? 2 : 1) * M * experts, K, 128, &wmap);
     if (rc) return rc;
-    constexpr size_t smem = 1024 + (size_t)GE_STAGES * GE_STAGE_BYTES + (2 * GE_STAGES + 2) * 8 + 16;
+    constexpr size_t smem = 1024 + (size_t)GE_STAGES * GE_STAGE_BYTES + (2 * GE_STAGES + 3) * 8 + 16;
     static bool configured = false;
     static int sms = 0;
     if (!configured) {

@@ -8,10 +8,11 @@ import pytest
 from mashbox_b200.ops.build import CSRC
 
 
-@pytest.mark.parametrize("source", ["gemm_f32_tc5.cu"])
+@pytest.mark.parametrize("source", ["gemm_f32_tc5.cu", "gemm_experts.cu"])
 def test_roles_wait_for_what_they_sent_for(source):
     text = open(os.path.join(CSRC, source)).read()
-    body = text[text.index("__global__ void __launch_bounds__", text.index("struct ")):text.index("// common exit")]
+    text = text[:text.index("// common exit")]
+    body = text[text.rindex("__global__"):]
     roles = re.split(r"\n {4,8}(?:\} else )?if \(warp (?:<|==|>=)", body)
     sends = [r for r in roles if re.search(r"tma_load_2d\(", r)]
     issues = [r for r in roles if re.search(r"umma_f16(_warp)?\(", r)]
