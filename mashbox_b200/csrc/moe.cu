@@ -699,7 +699,7 @@ MB_API int mb_moe_grouped_bf16(const void* h, const int* ids, const void* wg, co
 // Steps of 128 tokens and more (bf16) hand the two products to gemm_experts.cu, which wants the rows of every expert side by
 // side, starting at a multiple of 128:
 //   moe_sort_padded   one block: per pair its row in that layout (`place`), per tile of 128 rows what starts there (`groups`:
-//                     expert | rows << 12 for up to 256 rows of an expert, -1: nothing)
+//                     expert | its rows from there on, up to 256, << 12 | whether an odd tile of its << 24; -1: nothing)
 //   moe_gather_rows   h rows, by token, to their places
 //   moe_combine_rows  out[n] = sum over the places, in order, of weight * y[place of (n, k)]
 __global__ void moe_sort_padded_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ place,
@@ -724,7 +724,8 @@ __global__ void moe_sort_padded_kernel(const int* __restrict__ ids, int P, int E
     for (int t = threadIdx.x; t < max_tiles; t += blockDim.x) groups[t] = -1;
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        for (int t = start[e]; t < start[e + 1] && t < max_tiles; t += 2) groups[t] = e | min(256, cnt[e] - (t - start[e]) * 128) << 12;
+        for (int t = start[e]; t < start[e + 1] && t < max_tiles; t++)
+            groups[t] = e | min(256, cnt[e] - (t - start[e]) * 128) << 12 | (t - start[e] & 1) << 24;
         cnt[e] = start[e] * 128;                    // from here on: the next free row of the expert
     }
     __syncthreads();

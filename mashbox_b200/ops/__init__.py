@@ -762,13 +762,30 @@ def moe_tc5_tiles(N, top, E):
     return N * top // 128 + E
 
 
+def moe_tc5_rows(rows, K, gated):
+    """-> 256 or 128, the most rows of an expert that a tile of its product takes (gemm_experts.cu), by the rows an expert has on
+    average and its K.  Tiles of 128 have two pairs of accumulators, so one is written out under the products of the next, and leave
+    fewer blocks idle at the end; a tile of 256 reads the weights once where two of 128 read them twice.  That pays where one tile
+    holds what two would, and with very many rows, where there are enough tiles for all and each is long.  us, gate and up of 64 of
+    which a token takes 8, tiles of 256 / 128, K 4,096, 2 x 2,048 features: 100 rows 360 / 352, 128 377 / 412, 190 419 / 467, 256 620 /
+    556; of 8, a token takes 4: 512 rows 159 / 119, 768 203 / 174, 1,024 209 / 228; K 2,048, 2 x 1,408: 512 64 / 51, 1,024 95 / 83;
+    K 7,168, 2 x 2,048: 640 263 / 250, 768 266 / 300.  Down, K 1,408, 2,048 features: 190 22 / 17, 512 41 / 27, 1,024 46 / 50;
+    K 2,048, 4,096 features, of 64: 190 228 / 261, 250 288 / 306."""
+    if rows <= (230 if gated or K < 2048 else 256):
+        return 256 if rows > 112 and K >= 1536 else 128
+    if gated:
+        return 256 if (rows >= 900 and K >= 3072) or (rows >= 700 and K >= 6144) else 128
+    return 256 if rows >= 900 and K >= 512 else 128
+
+
 def moe_tc5(h, ids, wts, wgu, wd, out, rows, act, y, scratch, limit, alpha, shift=1.0, shared=None, gate=None,
-            row_scale=None):
+            row_scale=None, most=None):
     """The routed experts of a step of many tokens, bf16: ids (N, top) and wts from moe_select; wgu (E, 2F, D), every
     expert's gate rows then its up rows; wd (E, D, F); out (N, D).  Working memory, with T = moe_tc5_tiles(N, top, E):
     rows (128 T, D) bf16, act (128 T, F) bf16, y (128 T, D) float32, scratch (N top + T) int32.  shared (N, D) and gate
     (float32, one logit per token, rows gate.stride(0) apart): see moe_combine.  row_scale (128 T float32, working memory): the
-    weights meet the experts' inputs instead of their outputs."""
+    weights meet the experts' inputs instead of their outputs.  most: (gate and up, down) 256 or 128 rows a tile; by the sizes when
+    None.  The results are the same bits."""
     _cuda(h, ids, wts, wgu, wd, out, rows, act, y, scratch, shared, gate, row_scale)
     N, D = h.shape
     E, F = wgu.shape[0], wgu.shape[1] // 2
@@ -777,17 +794,19 @@ def moe_tc5(h, ids, wts, wgu, wd, out, rows, act, y, scratch, limit, alpha, shif
     if rows.shape[0] < 128 * T or act.shape[0] < 128 * T or y.shape[0] < 128 * T or scratch.numel() < N * top + T \
             or (row_scale is not None and row_scale.numel() < 128 * T):
         raise KernelError("moe_tc5: the working memory is too small")
+    if most is None:
+        most = moe_tc5_rows(N * top / E, D, True), moe_tc5_rows(N * top / E, F, False)
     place, groups = scratch[:N * top], scratch[N * top:N * top + T]
     f = _fn("moe", "mb_moe_sort_gather", [c_void_p] * 5 + [c_int] * 4 + [c_void_p] * 3)
     _check(f(_p(h), _p(ids), _p(place), _p(groups), _p(rows), N, D, E, top, _p(wts), _p(row_scale), _stream()),
            "moe_sort_gather")
     err = error_word(h.device)
     f = _fn("gemm_experts", "mb_gemm_experts_gated_bf16",
-            [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_int, c_float, c_float, c_float, c_void_p, c_void_p, c_void_p])
-    _check(f(_p(rows), _p(wgu), _p(act), 128 * T, F, D, _p(groups), E, float(limit), float(alpha), float(shift),
+            [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_int, c_int, c_float, c_float, c_float, c_void_p, c_void_p, c_void_p])
+    _check(f(_p(rows), _p(wgu), _p(act), 128 * T, F, D, _p(groups), E, most[0], float(limit), float(alpha), float(shift),
              _p(row_scale), _p(err), _stream()), "gemm_experts_gated")
-    f = _fn("gemm_experts", "mb_gemm_experts_f32out", [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_int, c_void_p, c_void_p])
-    _check(f(_p(act), _p(wd), _p(y), 128 * T, D, F, _p(groups), E, _p(err), _stream()), "gemm_experts")
+    f = _fn("gemm_experts", "mb_gemm_experts_f32out", [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_int, c_int, c_void_p, c_void_p])
+    _check(f(_p(act), _p(wd), _p(y), 128 * T, D, F, _p(groups), E, most[1], _p(err), _stream()), "gemm_experts")
     f = _fn("moe", "mb_moe_combine_rows", [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_void_p, c_int, c_void_p])
     _check(f(_p(y), _p(place), _p(wts if row_scale is None else None), _p(out), N, D, top, _p(shared), _p(gate), gate.stride(0) if gate is not None else 0,
              _stream()), "moe_combine_rows")
