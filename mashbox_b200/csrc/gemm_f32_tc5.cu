@@ -145,12 +145,52 @@ template <int HALF, int TN> __device__ __forceinline__ void fs_add_small(uint32_
     }
 }
 
-__device__ __noinline__ float fs_plain_chain(const float* a, const float* w, int K) {
-    float s = 0.0f;
-    for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
-    return s;
-}
 __device__ __forceinline__ bool fs_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u; }
+
+// The results of a block's tile that are not finite, as chains of fused multiply-adds in ascending k: `odd` has a bit for every column
+// that holds one.  The whole block goes through them, 32 columns at a time, operands staged in shared memory (buf); a thread has a row of
+// W and eight columns.  (A thread by itself for each such result made 509 rows of NaN x 16384 x 2048 take 71 ms, now 4.1; one such row 0.62.)
+__device__ __noinline__ void fs_chains(float* buf, const uint32_t* odd, int words, const float* __restrict__ A, const float* __restrict__ W,
+                                       float* C, int M, int K, int ldc, int tok0, int m0) {
+    constexpr int PITCH = 36;                                  // floats of a staged row of 32: 16-byte reads of 8 rows side by side
+    float *ws = buf, *as = buf + 128 * PITCH;
+    int *list = reinterpret_cast<int*>(as + 32 * PITCH), count = 0;
+    for (int i = 0; i < words; i++)
+        for (uint32_t left = odd[i]; left; left &= left - 1, count++)
+            if (threadIdx.x == 0) list[count] = i * 32 + __ffs(left) - 1;
+    const int r = threadIdx.x & 127, g = threadIdx.x >> 7;
+    for (int base = 0; base < count; base += 32) {
+        float acc[8] = {};
+        for (int k0 = 0; k0 < K; k0 += 32) {
+            __syncthreads();
+            for (int e = threadIdx.x; e < 128 * 8; e += FS_THREADS) {
+                const int row = e >> 3, k = (e & 7) * 4;
+                if (m0 + row < M && k0 + k < K)
+                    *reinterpret_cast<float4*>(ws + row * PITCH + k) = *reinterpret_cast<const float4*>(W + (size_t)(m0 + row) * K + k0 + k);
+            }
+            for (int e = threadIdx.x; e < 32 * 32; e += FS_THREADS) {
+                const int col = e >> 5, k = e & 31;
+                if (base + col < count && k0 + k < K) as[col * PITCH + k] = A[(size_t)(tok0 + list[base + col]) * K + k0 + k];
+            }
+            __syncthreads();
+            const int depth = min(32, K - k0);                  // a multiple of 4
+            for (int k = 0; k < depth; k += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(ws + r * PITCH + k);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float4 a = *reinterpret_cast<const float4*>(as + (g * 8 + j) * PITCH + k);
+                    acc[j] = fmaf(a.w, w.w, fmaf(a.z, w.z, fmaf(a.y, w.y, fmaf(a.x, w.x, acc[j]))));
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (m0 + r < M && base + g * 8 + j < count) {
+                float* p = C + (size_t)(tok0 + list[base + g * 8 + j]) * ldc + m0 + r;
+                if (!fs_finite(*p)) *p = acc[j];
+            }
+    }
+}
 
 __device__ __forceinline__ float fs_ld_cluster(uint32_t addr, int rank) {
     uint32_t at;
@@ -175,7 +215,8 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
     const uint32_t stage0 = smem_u32(smem), raw0 = stage0 + S::STAGES * S::STAGE;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::STAGES * S::STAGE + FS_RAW * FS_RAW_BYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t*>(bars + 32), *odd = tmem_slot + 1;
+    constexpr int ODD = (TN + 31) / 32;                        // a bit for every column of the tile with a result that is not finite
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * S::STAGES, rfull0 = empty0 + 8 * S::STAGES,
                    rempty0 = rfull0 + 8 * FS_RAW, tfull0 = rempty0 + 8 * FS_RAW, sfull = tfull0 + 16, sempty = sfull + 8,
                    xfull0 = sempty + 8, done = xfull0 + 8 * S::STAGES;
@@ -188,6 +229,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         for (int a = 0; a < 2; a++) mbar_init(tfull0 + 8 * a, 1);
         mbar_init(sfull, 1);
         mbar_init(done, 1);
+        for (int i = 0; i < ODD; i++) odd[i] = 0;
         mbar_init(sempty, 8);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -310,7 +352,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         for (int j = 0; j < HALF; j++) sum[j] = 0.0f;
         float* out = C + (size_t)(tok0 + half * HALF) * ldc + m;
         const int cols = m < M ? min(HALF, N - tok0 - half * HALF) : 0;        // columns this thread has (0 or less: none)
-        bool ok = true, odd = false;
+        bool some = false;
         int at = 0, periods = 0;                                // as the products count them
         // an accumulator that has been read is among the arrivals that the products of the block after the next wait for
         if (lane == 0) {
@@ -321,7 +363,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         for (int i = 0; i < nb; i++) {
             const int acc = i & 1;
             bool got = mbar_wait(tfull0 + 8 * acc, (i >> 1) & 1, err);
-            if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, got)) break;
             tc_fence_after();
             fs_add<HALF>(taddr + acc * TN, at == 0, sum);
             tc_fence_before();
@@ -331,7 +373,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             const bool ends = at == quarter || i + 1 == nb;
             if (ends || at % FS_PERIOD == 0) {
                 got = mbar_wait(sfull, periods & 1, err);
-                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, got)) break;
                 periods++;
                 tc_fence_after();
                 fs_add_small<HALF, TN>(taddr + 2 * TN, sum);
@@ -359,17 +401,16 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                         const float v = start ? sum[c + j] : before[j] + sum[c + j];
                         if (c + j < cols) {
                             p[(size_t)j * step] = v;
-                            if (last) odd |= !fs_finite(v);
+                            if (last) some |= !fs_finite(v);
                         }
                     }
                 }
             }
             if (at == quarter) at = 0;
         }
-        if (CL == 1 && ok && odd) {
+        if (CL == 1 && some) {
             for (int c = 0; c < cols; c++)
-                if (!fs_finite(out[(size_t)c * ldc]))
-                    out[(size_t)c * ldc] = fs_plain_chain(A + (size_t)(tok0 + half * HALF + c) * K, W + (size_t)m * K, K);
+                if (!fs_finite(out[(size_t)c * ldc])) atomicOr(odd + (half * HALF + c) / 32, 1u << ((half * HALF + c) % 32));
         }
         if (CL > 1) {
             // every product and copy of this block is done: its sums go where the stages lay, a row of 128 for every column
@@ -392,7 +433,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                     v = b == 0 ? x : v + x;
                 }
                 if (n < N && m < M) {
-                    if (!fs_finite(v)) v = fs_plain_chain(A + (size_t)n * K, W + (size_t)m * K, K);
+                    if (!fs_finite(v)) atomicOr(odd + (c0 + c) / 32, 1u << ((c0 + c) % 32));
                     C[(size_t)n * ldc + m] = v;
                 }
             }
@@ -407,6 +448,10 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         tc_fence_after();
         tmem_dealloc(tmem_base, S::TMEM);
     }
+    uint32_t any = 0;
+#pragma unroll
+    for (int i = 0; i < ODD; i++) any |= odd[i];
+    if (any) fs_chains(reinterpret_cast<float*>(smem), odd, ODD, A, W, C, M, K, ldc, tok0, m0);
 }
 
 // ------------------------------------------------------------------------------------------------ host side
