@@ -1,6 +1,6 @@
 // True 32-bit matrix product for the float32 path on the FMA units: C[n, m] = sum_k A[n, k] * W[m, k], no tensor cores, no
-// TF32.  It takes the matrices gemm_f32_tc5.cu does not (fewer than 64 rows or 128 columns, rows off 16-byte boundaries), whatever
-// the number of rows of A.
+// TF32.  It takes the matrices that do not go to gemm_f32_tc5.cu (ops.f32_split_supports: fewer than 64 rows, a short K, rows off
+// 16-byte boundaries), whatever the number of rows of A.
 // Every output element is one float accumulator fed by fused multiply-adds in ascending k, so its value depends on neither
 // the number of rows in the call nor on the tile it falls into: the 32-bit path gives the same logits however the tokens
 // are cut into steps.

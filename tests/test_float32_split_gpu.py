@@ -210,3 +210,14 @@ def test_a_prompt_of_nan_costs_a_few_products():
         return best
     plain = took(a)
     assert took(torch.full_like(a, float("nan"))) < 40 * plain and bool(torch.isnan(out).all())
+
+
+@pytest.mark.parametrize("N,M,Kd,split", [(33, 512, 128, False), (5, 2048, 192, False), (300, 161, 252, False), (7, 160, 128, True),
+                                          (20, 161, 256, True), (9, 63, 512, False), (9, 64, 258, False)])
+def test_short_matrices_stay_on_the_fma_units(N, M, Kd, split):
+    """where the tensor cores' two launches cost more (ops.f32_split_supports): the same bits as the FMA units' product"""
+    K = ops()
+    a, w = operands(N, M, Kd)
+    assert K.f32_split_supports(w) == split
+    want = K.linear_f32_split(a, w, torch.empty(N, M, device=G.DEV)) if split else chain(a, w)
+    assert torch.equal(K.linear(a, w), want)
