@@ -486,6 +486,32 @@ static int fs_launch(const CUtensorMap& wmap, const float* A, const float* W, fl
     return 0;
 }
 
+// blocks the device holds at once, and clusters of four of them (a block fills an SM): asked for once, on the device of the first call
+struct FsSlots { int blocks, clusters; };
+static FsSlots fs_ask() {
+    FsSlots s = {148, 35};
+    int dev = 0, sms = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        return s;
+    s = {sms, sms / 4 > 2 ? sms / 4 - 2 : 1};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 4;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(4);
+    cfg.blockDim = dim3(FS_THREADS);
+    cfg.dynamicSmemBytes = FsShape<128>::SMEM;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(gemm_f32_tc5_kernel<128, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, FsShape<128>::SMEM) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, gemm_f32_tc5_kernel<128, 4>, &cfg) == cudaSuccess && n > 0)
+        s.clusters = n;
+    else
+        cudaGetLastError();
+    return s;
+}
+
 // The tile: rows of A a block, and whether a cluster shares K.  Cost of a choice = rounds of blocks x (stages x time of a stage +
 // what a block costs beside them), both as measured (one tile size alone on 2,048 and 8,192 k; the sums of the quarters through C
 // are in it).  us, 64 alone / 128 alone / 128 in fours: 509 x 16384 x 2048 350 / 258 / 357, 509 x 2048 x 2048 55 / 67 / 50, 509 x 2048 x
@@ -495,11 +521,12 @@ static void fs_choose(int N, int M, int K, int* tn, int* cl) {
     static const int TNS[4] = {16, 32, 64, 128};
     static const int STAGE_NS[4][2] = {{575, 575}, {630, 600}, {680, 650}, {740, 760}};
     static const int BLOCK_NS[4][2] = {{4000, 6000}, {5000, 6000}, {9000, 7000}, {16000, 10000}};
+    static const FsSlots held = fs_ask();
     const long long blocks = (K + FS_BK - 1) / FS_BK, quarter = (blocks + 3) / 4, rows = (M + 127) / 128;
     long long best = -1;
     for (int i = 0; i < 4; i++)
         for (int c = 0; c < 2; c++) {
-            const long long units = rows * ((N + TNS[i] - 1) / TNS[i]), slots = c ? 35 : 148;          // tiles the device holds at once
+            const long long units = rows * ((N + TNS[i] - 1) / TNS[i]), slots = c ? held.clusters : held.blocks;
             const long long cost = (units + slots - 1) / slots * ((c ? quarter : blocks) * STAGE_NS[i][c] + BLOCK_NS[i][c]);
             if (best < 0 || cost < best) { best = cost; *tn = TNS[i]; *cl = c ? 4 : 1; }
         }
