@@ -74,7 +74,7 @@ class ModelRunner:
                 raise RequestError("the step has tokens to be filled in on the device, but no sampled ids were given")
             kernels.patch_tokens(self.inputs.get("token_ids"), sampled, pairs, pairs.numel() // 2)
         self.cache.flush_tables()
-        logits = self._run_graph(ctx) if self.use_graphs else self.model.forward(ctx)
+        logits = self._run_graph(ctx) if self.use_graphs else self._forward(ctx)
         self.commit(entries)
         return logits if logits is None or ctx.real_out == ctx.n_out else logits[:ctx.real_out]
 
@@ -187,6 +187,15 @@ class ModelRunner:
             self.stats["tokens"] += len(tokens)
         self.stats["steps"] += 1
 
+    def _forward(self, ctx):
+        with kernels.float32_planes(self._float32_planes):
+            return self.model.forward(ctx)
+
+    def _float32_planes(self, rows, most, Kp):
+        """the float32 products' working memory, one buffer for all of a step, made for the largest"""
+        values = 3 * max(rows, min(self.ws.max_rows, most)) * Kp
+        return self.ws.get("float32_planes", values, (), torch.bfloat16, reserve=values)
+
     def _run_graph(self, ctx):
         sig = (self.inputs.signature(), getattr(self.ws, "generation", 0), getattr(self.inputs, "generation", 0),
                kernels.scratch_generation())
@@ -199,7 +208,7 @@ class ModelRunner:
         count = self.seen_signatures.get(sig, 0)
         self.seen_signatures[sig] = count + 1
         if count == 0:                      # first time: run eagerly (loads kernels, sizes buffers)
-            return self.model.forward(ctx)
+            return self._forward(ctx)
         # Captured on a stream of its own that first waits for the step's stream; the GPU goes on with the steps it
         # has queued meanwhile (no device-wide wait, no emptying of the allocator's cache).
         t0 = time.perf_counter()
@@ -223,7 +232,7 @@ class ModelRunner:
             with torch.cuda.stream(self.capture_stream):
                 graph.capture_begin(pool=self.graph_pool, capture_error_mode="thread_local")
                 try:
-                    logits = self.model.forward(ctx)
+                    logits = self._forward(ctx)
                 except BaseException:
                     try:
                         graph.capture_end()

@@ -5,8 +5,10 @@ refuses the sizes.  There is no CPU or library fallback for a kernel: if the ext
 there, the call fails.  The only library call is the bf16 matrix product (cuBLAS through torch.mm), which stands where
 the reference engine, too, hands its contractions to a library (src/mashbox/ops/dense16.py:73-75).
 """
+import contextlib
 import ctypes
 import functools
+import threading
 
 import torch
 
@@ -881,7 +883,22 @@ def f32_split_supports(w):
     return K % 4 == 0 and (K >= 256 or (K >= 128 and M <= 160)) and M >= 64 and w.data_ptr() % 16 == 0
 
 
-F32_SPLIT_PLANE = 1 << 26          # values of a plane of a's bf16 parts (three planes, 6 bytes a value): more rows go in slabs
+# values of a plane of a's bf16 parts (three planes, 6 bytes a value: 100 MB; 2,048 rows of 8,192): more rows go in slabs
+F32_SPLIT_PLANE = 1 << 24
+_float32_planes = threading.local()
+
+
+@contextlib.contextmanager
+def float32_planes(buffer):
+    """Within it float32 products of this thread take the memory of their operand's parts from buffer(rows, most, Kp), a flat
+    bfloat16 tensor of at least 3 rows Kp values on the operand's device (most: the rows a product asks for at a time at most);
+    outside of it a product allocates it.  For one stream: the products of a step use it one after the other."""
+    before = getattr(_float32_planes, "buffer", None)
+    _float32_planes.buffer = buffer
+    try:
+        yield
+    finally:
+        _float32_planes.buffer = before
 
 
 def linear_f32_split(a, w, out, tile=0, cluster=0):
@@ -891,7 +908,9 @@ def linear_f32_split(a, w, out, tile=0, cluster=0):
     N, K = a.shape
     M, Kp = w.shape[0], (K + 7) // 8 * 8
     most = max(256, F32_SPLIT_PLANE // Kp)
-    planes = torch.empty((3 * min(N, most), Kp), dtype=torch.bfloat16, device=a.device)
+    buffer = getattr(_float32_planes, "buffer", None)
+    planes = buffer(min(N, most), most, Kp) if buffer is not None else \
+        torch.empty(3 * min(N, most) * Kp, dtype=torch.bfloat16, device=a.device)
     f = _fn("gemm_f32_tc5", "mb_gemm_f32_tc5", [c_void_p] * 4 + [c_int] * 6 + [c_void_p] * 2)
     for lo in range(0, N, most):
         n = min(N, lo + most) - lo
