@@ -5,8 +5,8 @@
 // the number of rows in the call nor on the tile it falls into: the 32-bit path gives the same logits however the tokens
 // are cut into steps.
 //
-// Bound by the FMA pipes for prompts (some 74 TFLOP/s: 148 SMs x 128 lanes; 50 reached on 509 x 16384 x 2048, 25 by a tile
-// of 4 x 4 a thread without a stage ahead), by memory and the latency of a stage for a handful of rows.  A thread owns
+// Bound by the FMA pipes for prompts (some 74 TFLOP/s: 148 SMs x 128 lanes; 50 reached on 509 x 16384 x 2048 with aligned rows, which
+// go to the tensor cores now, 45 with K 2,050), by memory and the latency of a stage for a handful of rows.  A thread owns
 // TM x TN outputs and works on pairs of neighbouring columns (fma.rn.f32x2: one issue slot, two results, each rounded as
 // the single one is), so that half of the issue slots are left for the reads of shared memory that feed them.  The operands
 // lie k by k in shared memory, two stages of BK; the next stage is in registers while the current one is worked through.
@@ -161,13 +161,12 @@ MB_API int mb_gemm_f32(const float* A, const float* W, float* C, int N, int M, i
     auto padded = [&](int bm) { return ((long long)N + bm - 1) / bm * bm; };
     auto tiles = [&](int bm, int bn) { return padded(bm) / bm * ((M + bn - 1) / bn); };
     // The largest tile that still gives every SM its four blocks, since it reads the operands least (64 rows of the first cost
-    // what 56 of the second do), unless its padding costs more than that; measured (us, 128 x 64 / 64 x 64 / 32 x 64 /
-    // 16 x 64): 509 x 16384 x 2048 688 / 770 / 966 / 1330; 160 x 32000 x 2048, where the first has 256 rows and the second
-    // 192, 674 / 606 / 629 / 817; 509 x 2048 x 2048, where the first leaves most SMs idle, 145 / 131 / 150 / 190; the head of
-    // 128,256 columns (K 2,048): 128 rows 1329 / 1511 / 1911 / 2593, 65 rows 1288 / 1468 / 1413 / 1599, 64 rows 1288 / 774 /
-    // 967 / 1332, 33 rows 1268 / 748 / 942 / 993, 32 rows 1266 / 748 / 496 / 678, 17 rows 1262 / 737 / 481 / 664, one row
-    // 1253 / 729 / 469 / 336; 17 x 16384 x 2048 219 / 129 / 109 / 111; 130 x 2048 x 2048 145 / 81 / 91 / 62.  (One tile of
-    // 64 x 64 for all, without a stage ahead: 1355, 1053, 227, 2678, 2464, 1360, 1257, 1257, 1206, 1158, 225, 156.)
+    // what 56 of the second do), unless its padding costs more than that; measured at sizes that come here (us, 128 x 64 / 64 x 64 /
+    // 32 x 64 / 16 x 64): a short K: 2,048 x 2,048 x 128 29 / 28 / 34 / 45, 2,048 x 8,192 x 192 131 / 149 / 185 / 252, 509 x 1,024 x 192
+    // 16 / 9.6 / 11 / 11, 64 x 2,048 x 128 11 / 6.9 / 6.7 / 4.8; few rows of W: 509 x 48 x 8,192 552 / 287 / 280 / 177; K no multiple of 4,
+    // in single loads: 509 x 16,384 x 2,050 755 / 985 / 1437 / 1884, 509 x 2,048 x 2,050 145 / 149 / 191 / 244, 160 x 32,000 x 2,050 731 /
+    // 759 / 927 / 1342, 64 rows 408 / 295 / 331 / 543, 33 rows 399 / 277 / 335 / 522, 17 rows 394 / 264 / 180 / 235, one 391 / 253 / 171 /
+    // 138.  (It costs up to 15 % where the first tile has nearly enough blocks: 128 x 32,000 x 2,050 444 / 509 / 742 / 1077.)
     const int t = N <= 16                                                        ? 3
                   : tiles(128, 64) >= 592 && 7 * padded(128) <= 8 * padded(64) ? 0
                   : N > 32 && tiles(64, 64) >= 148                             ? 1
