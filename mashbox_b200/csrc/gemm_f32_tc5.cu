@@ -12,12 +12,12 @@
 // 1.0e-7 / 1.6e-7 at K 512 / 2,048 / 8,192 on normal values, the chain's 4e-7 / 8e-7 / 16e-7; measured by the sum of the products'
 // magnitudes the worst element is nearer too, but where two to a few products of one block of 32 decide a result, what h h is cut
 // off by (up to 2^-23) beside the last rounding is some 1.6 times the chain's few roundings (tests/test_float32_split_gpu.py).
-// (With h h in one accumulator with the rest and m l, l m left out, up to 2^-22 of a product was missing; a block was 12 instructions then,
-// not 10, but 256 rows of A fitted: 509 x 2048 x 2048 37 us, now 49.)  Bound by the chain of a stage: 0.73 us with 128 rows of A, 0.58
-// with 2 of its 10 instructions, 0.51 without the cutting besides; more stages of either ring bring nothing.  W's planes in tensor
-// memory, so that the instructions read half as much shared memory, 0.97 (16 instructions).  The FMA units' product at the same size
-// and this one, us: 509 x 16384 x 2048 684 and 251, 509 x 2048 x 8192 491 and 126, 509 x 2048 x 2048 123 and 49, one row x 2048 x
-// 2048 97 and 17.
+// (With h h in one accumulator with the rest and m l, l m left out, up to 2^-22 of a product was missing; a block was 12 instructions
+// then, not 10, but 256 rows of A fitted: 509 x 2048 x 2048 37 us, now 48.)  Bound by the chain of a stage: 0.73 us with 128 rows of A,
+// tensor pipes busy 0.59 of it; before the products waited on one barrier alone 0.77, 0.58 with 2 of the 10 instructions, 0.51 without
+// the cutting besides; more stages of either ring bring nothing.  W's planes in tensor memory, so that the instructions read half
+// as much shared memory, 0.97 (16 instructions, two waits).  The FMA units' product at the same size and this one, us: 509 x 16384 x
+// 2048 684 and 247, 509 x 2048 x 8192 491 and 119, 509 x 2048 x 2048 123 and 48, one row x 2048 x 2048 97 and 18.
 //
 // An output is the same operations in the same order however many rows a call has: blocks of 32 k in ascending order
 // within a quarter of K, the quarters' sums in ascending order.  Tiles, and whether one block or a cluster of four goes
@@ -28,14 +28,16 @@
 //   warp 2      TMA: the three bf16 planes of TN x 32 values of A (64-byte swizzle), cut by split_rows_kernel beforehand:
 //               they are read once per tile of W, W once per tile of A
 //   warps 4-7   cut a stage of W into its three planes in shared memory, as the instructions want them
-//   warp 3      tells the products' barrier that planes have come
-//   warp 1      one lane issues the products; accumulators of TN columns, two in turn
-//   warps 8-15  add a block's accumulator to the sums in registers (thread = a row of W, half of the columns)
+//   warp 3      tells the products' barrier that planes of A have come
+//   warp 1      one lane issues the products; accumulators of TN columns, two in turn for h h, two side by side for the rest
+//   warps 8-15  add the accumulators to the sums in registers (thread = a row of W, half of the columns)
 // A cluster of four blocks takes a quarter of K each where the tiles alone leave the device idle: the sums meet in
 // shared memory.  A single block puts the sum of a quarter down in C and adds the next to it.
 //
-// A result that is not finite is computed again as one chain of fused multiply-adds, so infinities and NaN come out as the
-// plain product has them (an infinite operand has no such parts).
+// A result that is not finite is computed again as one chain of fused multiply-adds (fs_chains), so infinities and NaN come out as
+// the plain product has them: an infinite operand has no such parts, and sums from 2^80 on overflow with the factors of 2^24.
+// The cut into three parts is that of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for
+// higher-precision computations" (2019).
 #include "tcgen05.cuh"
 
 MB_PDL_SWITCH(mb_gemm_f32_tc5_set_pdl)              // the product starts, and brings W in, while the planes are cut
@@ -514,9 +516,9 @@ static FsSlots fs_ask() {
 
 // The tile: rows of A a block, and whether a cluster shares K.  Cost of a choice = rounds of blocks x (stages x time of a stage +
 // what a block costs beside them), both as measured (one tile size alone on 2,048 and 8,192 k; the sums of the quarters through C
-// are in it).  us, 64 alone / 128 alone / 128 in fours: 509 x 16384 x 2048 350 / 258 / 357, 509 x 2048 x 2048 55 / 67 / 50, 509 x 2048 x
-// 8192 189 / 218 / 128, 509 x 3072 x 2048 102 / 67 / 72, 300 x 16384 x 2048 247 / 194 / 270, 64 x 2048 x 256 14 / 20 / 13 (32 in fours 8.4);
-// one row x 2048 x 2048: 16 alone 45, in fours 17.
+// are in it).  us, 64 alone / 128 alone / 128 in fours: 509 x 16384 x 2048 340 / 247 / 350, 509 x 2048 x 2048 54 / 64 / 48, 509 x 2048 x
+// 8192 183 / 202 / 119, 509 x 3072 x 2048 99 / 65 / 69, 300 x 16384 x 2048 237 / 188 / 257, 64 x 2048 x 256 14 / 20 / 13 (32 in fours
+// 8.6); one row x 2048 x 2048: 16 alone 47, in fours 18.
 static void fs_choose(int N, int M, int K, int* tn, int* cl) {
     static const int TNS[4] = {16, 32, 64, 128};
     static const int STAGE_NS[4][2] = {{575, 575}, {630, 600}, {680, 650}, {740, 760}};
