@@ -427,6 +427,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         if (warp >= 8) {
             constexpr int MINE = TN / CL;                       // columns this block adds up
             const int r = tid & 127, m = m0 + r, c0 = rank * MINE;
+            bool some = false;
             for (int c = (tid - 256) >> 7; c < MINE; c += 2) {
                 const int n = tok0 + c0 + c;
                 float v = 0.0f;
@@ -435,10 +436,14 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                     v = b == 0 ? x : v + x;
                 }
                 if (n < N && m < M) {
-                    if (!fs_finite(v)) atomicOr(odd + (c0 + c) / 32, 1u << ((c0 + c) % 32));
+                    some |= !fs_finite(v);
                     C[(size_t)n * ldc + m] = v;
                 }
             }
+            if (some)
+                for (int c = (tid - 256) >> 7; c < MINE; c += 2)
+                    if (tok0 + c0 + c < N && m < M && !fs_finite(C[(size_t)(tok0 + c0 + c) * ldc + m]))
+                        atomicOr(odd + (c0 + c) / 32, 1u << ((c0 + c) % 32));
         }
         __syncwarp();
         fs_cluster_sync();                                      // nobody leaves while its sums are read
@@ -516,7 +521,7 @@ static FsSlots fs_ask() {
 
 // The tile: rows of A a block, and whether a cluster shares K.  Cost of a choice = rounds of blocks x (stages x time of a stage +
 // what a block costs beside them), both as measured (one tile size alone on 2,048 and 8,192 k; the sums of the quarters through C
-// are in it).  us, 64 alone / 128 alone / 128 in fours: 509 x 16384 x 2048 340 / 247 / 350, 509 x 2048 x 2048 54 / 64 / 48, 509 x 2048 x
+// are in it).  us, 64 alone / 128 alone / 128 in fours: 509 x 16384 x 2048 340 / 247 / 338, 509 x 2048 x 2048 54 / 64 / 48, 509 x 2048 x
 // 8192 183 / 202 / 119, 509 x 3072 x 2048 99 / 65 / 69, 300 x 16384 x 2048 237 / 188 / 257, 64 x 2048 x 256 14 / 20 / 13 (32 in fours
 // 8.6); one row x 2048 x 2048: 16 alone 47, in fours 18.
 static void fs_choose(int N, int M, int K, int* tn, int* cl) {
